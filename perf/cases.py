@@ -286,8 +286,8 @@ def _batch_table(case, seed):
 
 def _batch_specs(t, case):
     """The case's queries (templates, slices, parameters): the same for every seed, over other data."""
-    return workload.random_queries(t, case["queries"], np.random.default_rng([case["rows"], case["queries"]]),
-                                   min_rows=1_000_000, ht_layout="linear")
+    return workload.random_queries(t, case["queries"], np.random.default_rng(case["queries"]), min_rows=1_000_000,
+                                   ht_layout="linear")
 
 
 def _prepare_batch(case, seed):

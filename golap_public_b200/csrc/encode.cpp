@@ -412,7 +412,7 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
     if (threads == 0) threads = std::max(1u, std::thread::hardware_concurrency());
     threads = std::min<uint32_t>(threads, std::max<uint32_t>(1, col->n_slots));
     std::vector<std::vector<uint8_t>> bufs(threads);
-    std::atomic<bool> overflow{false};
+    std::atomic<bool> overflow{false}, all_simple{codec == GX_CODEC_CASCADED};
     std::vector<std::vector<uint64_t>> local_off(threads);
     auto work = [&](uint32_t t) {
         uint32_t s0 = (uint32_t)((uint64_t)col->n_slots * t / threads);
@@ -462,6 +462,11 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
                 buf.insert(buf.end(), lz4_tmp.begin(), lz4_tmp.end());
             } else {
                 used = casc_encode_block(vals + r0, rows, rle, delta, bp, buf, &col->seg[(size_t)2 * S * s]);
+                for (uint32_t p = 0; p * kCascPageRows < rows; ++p) {
+                    casc_hdr h;
+                    std::memcpy(&h, buf.data() + start + col->seg[(size_t)2 * S * s + 2 * p], sizeof(h));
+                    if (!casc_page_simple(h.flags, h.n_runs, h.val_bits, h.val_base)) all_simple = false;
+                }
             }
             buf.resize((buf.size() + kPayloadAlign - 1) & ~(size_t)(kPayloadAlign - 1), 0);
             col->blocks[s].offset = start;  // local, fixed up below
@@ -474,6 +479,7 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
     for (uint32_t t = 1; t < threads; ++t) pool.emplace_back(work, t);
     work(0);
     for (auto& th : pool) th.join();
+    col->casc_simple = all_simple;
     if (overflow) return set_error(GX_ERR_INVALID, "an LZ4 block exceeds the %u-byte staging buffer", kStageBytes);
     // the per-thread buffers in thread order, each copied by its own thread
     std::vector<uint64_t> shift(threads + 1, 0);

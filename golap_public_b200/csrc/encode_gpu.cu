@@ -450,6 +450,7 @@ extern "C" gx_status gx_column_encode_device(const int32_t* values_dev, uint64_t
         std::vector<uint64_t> offset(n_slots, 0);
         std::vector<uint32_t> page_off(codec == GX_CODEC_CASCADED ? (size_t)n_slots * (pages + 1) : 0, 0);
         uint64_t cursor = 0;
+        bool simple = codec == GX_CODEC_CASCADED;
         for (uint32_t sl = 0; sl < n_slots; ++sl) {
             const uint32_t c = sl / col->blocks_per_chunk, j = sl % col->blocks_per_chunk;
             const uint64_t c0 = (uint64_t)c * rpc, c1 = std::min<uint64_t>(n_rows, c0 + rpc);
@@ -484,7 +485,9 @@ extern "C" gx_status gx_column_encode_device(const int32_t* values_dev, uint64_t
                 uint32_t* po = &page_off[(size_t)sl * (pages + 1)];
                 uint32_t off = (8 + 4 * (n_pages + 1) + 15) & ~15u;
                 for (uint32_t p = 0; p < n_pages; ++p) {
-                    const uint32_t b = plans[(size_t)sl * pages + p].bytes;
+                    const PagePlan& pl = plans[(size_t)sl * pages + p];
+                    const uint32_t b = pl.bytes;
+                    if (!casc_page_simple(pl.flags, pl.n, pl.vbits, pl.vbase)) simple = false;
                     po[p] = off;
                     col->seg[(size_t)2 * S * sl + 2 * p] = off;
                     col->seg[(size_t)2 * S * sl + 2 * p + 1] = b;
@@ -506,6 +509,7 @@ extern "C" gx_status gx_column_encode_device(const int32_t* values_dev, uint64_t
             col->mins[c] = mn;
             col->maxs[c] = mx;
         }
+        col->casc_simple = simple;
         col->n_blocks = 0;
         for (auto& b : col->blocks) col->n_blocks += b.n_rows ? 1 : 0;
 

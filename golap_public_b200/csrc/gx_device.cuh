@@ -99,15 +99,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* m, uint32_t phase) {
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
-// L2 cache policies: join tables stay (evict last), streamed bytes go first.
+// L2 cache policy of join tables: they stay (evict last).
 __device__ __forceinline__ uint64_t ws_policy_keep() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ uint64_t ws_policy_stream() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
 // A join-table slot read under policy pol (read-only path).

@@ -76,6 +76,7 @@ constexpr uint32_t kCascMaxRuns = 2048;        // run tables of one decode (>= k
 constexpr uint32_t kCascPageLog2 = 11;
 constexpr uint32_t kCascPageRows = 1u << kCascPageLog2;  // rows of one cascaded page
 constexpr uint32_t kCascPageMaxRuns = 512;     // RLE pages hold at most this many runs
+constexpr uint32_t kCascFewRuns = 8;           // RLE pages of at most this many runs are scanned without a decode
 constexpr uint32_t kCascMaxPages = kMaxRowsPerBlock / kCascPageRows;
 constexpr uint32_t kStageBytes = 66048;        // shared staging buffer for one compressed block
 constexpr uint32_t kPayloadAlign = 16;
@@ -99,6 +100,13 @@ struct casc_hdr {
     uint32_t lens_off;   // byte offset of the length stream (0 without RLE)
 };
 static_assert(sizeof(casc_hdr) == 32, "casc_hdr layout");
+
+// A page the warp-tile scan evaluates from its own bytes: bit-packed values
+// without RLE or DELTA, one value, or a few runs.
+GX_HOSTDEV inline bool casc_page_simple(uint32_t flags, uint32_t n_runs, uint32_t val_bits, int32_t val_base) {
+    if (flags & CASC_RLE) return n_runs <= kCascFewRuns;
+    return !(flags & CASC_DELTA) || (val_bits == 0 && val_base == 0);
+}
 
 // Device block descriptor (16 bytes).
 struct gx_dblock {
@@ -180,6 +188,7 @@ struct gx_column {
     uint32_t* d_bloom = nullptr;
     // LZ4: every block is one 16-byte aligned literal run (-1 = not known yet)
     mutable int lz4_direct = -1;
+    bool casc_simple = false;  // cascaded: every page is simple (casc_page_simple), known when encoded
     int32_t* d_bmins = nullptr;
     int32_t* d_bmaxs = nullptr;
     int device = -1;

@@ -2198,12 +2198,23 @@ static bool lz4_all_direct(const gx_column* c) {
     return ok;
 }
 
+// Multiplier and shift with n / d == (uint64_t)n * mul >> shift for every
+// n < 2^31: shift = 31 + ceil(log2 d), mul = ceil(2^shift / d) (below 2^32,
+// as d > 2^(ceil(log2 d) - 1); the excess mul * d - 2^shift is below d <=
+// 2^(shift - 31), so it never carries a quotient over for n < 2^31).
+static void ws_divisor(uint32_t d, uint32_t* mul, uint32_t* shift) {
+    const uint32_t sh = 31 + log2_ceil(d);
+    *mul = (uint32_t)(((1ull << sh) + d - 1) / d);
+    *shift = sh;
+}
+
 // The warp-tile scan (warp_scan_kernel) for a plan, or *done = false when
 // the plan is not of its shape: HBM-resident (or staged) columns sharing the
 // table layout, LZ4 ones segmented with segments of at most kWsTile rows, no
-// BUILD, at most 32768 chunks.  Shared memory per warp: one kWsTile-row area
-// per column (a stage area for raw and all-literal LZ4 columns, a decode
-// buffer for cascaded and other LZ4 columns) and a group table for grouped
+// BUILD, at most 32768 chunks.  Shared memory per warp: its records and one
+// kWsTile-row decode buffer per match-bearing LZ4 column and per cascaded
+// column with pages that need a decode (raw and all-literal LZ4 columns and
+// simple cascaded pages are read in place); per CTA a group table for grouped
 // plans.
 static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd, const gx_column* c0, cudaStream_t s,
                                   unsigned long long* rows_dev, bool* done, const PipeGroup* grp = nullptr) {
@@ -2216,7 +2227,8 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     if (!shared_query(*plan, qd, cols, P.q, &why)) return GX_OK;
     if (cols.size() > kWsMaxCols) return GX_OK;
     uint32_t areas = 0;
-    for (size_t i = 0; i < kWsMaxCols; ++i) P.stage_of[i] = P.buf_of[i] = kWsNone;
+    bool cut_tiles = true;  // parts of a tile would each decode the whole tile's LZ4 segments
+    for (size_t i = 0; i < kWsMaxCols; ++i) P.buf_of[i] = kWsNone;
     for (size_t i = 0; i < cols.size(); ++i) {
         const gx_column* c = cols[i];
         const uint8_t* staged = nullptr;
@@ -2230,10 +2242,11 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
             P.cols[i].payload = staged;
             P.cols[i].host_mapped = 0;
         }
-        if (c->codec == GX_CODEC_NONE || (c->codec == GX_CODEC_LZ4 && lz4_all_direct(c)))
-            P.stage_of[i] = areas++;
-        else
+        if (!(c->codec == GX_CODEC_NONE || (c->codec == GX_CODEC_LZ4 && lz4_all_direct(c)) ||
+              (c->codec == GX_CODEC_CASCADED && c->casc_simple))) {
             P.buf_of[i] = areas++;
+            if (c->codec == GX_CODEC_LZ4) cut_tiles = false;
+        }
     }
     P.q.keep_in = plan->keep_chunks_dev;
     P.q.keep_out = plan->keep_out_dev;
@@ -2242,6 +2255,10 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     P.rows_per_chunk = c0->rows_per_chunk;
     P.rows_per_block = c0->rows_per_block;
     P.tiles_per_block = (c0->rows_per_block + kWsTile - 1) / kWsTile;
+    ws_divisor(P.blocks_per_chunk * P.tiles_per_block, &P.pc_mul, &P.pc_shift);
+    ws_divisor(P.tiles_per_block, &P.tpb_mul, &P.tpb_shift);
+    P.parts = cut_tiles ? 1u : 0u;
+    P.col_log2 = P.n_cols <= 4 && P.q.n_steps <= 4 && P.q.n_prune <= 4 ? 2u : 3u;
     P.n_rows = c0->n_rows;
     P.chunk_lo = grp ? grp->chunk_lo : 0u;
     P.chunk_hi = grp ? grp->chunk_hi : c0->n_chunks;
@@ -2268,10 +2285,7 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     else if (sig == kSigQ2) kern = warp_scan_kernel<kSigQ2>;
     else if (sig == kSigQ3) kern = warp_scan_kernel<kSigQ3>;
     else if (sig == kSigQ4) kern = warp_scan_kernel<kSigQ4>;
-    // shared memory per warp: the areas, then (grouped) the run-time
-    // evaluator's per-row group keys and the group table
-    const bool rt_eval = kern == warp_scan_kernel<0>;
-    P.warp_words = kWsHead + areas * kWsTile + (P.grouped_tab && rt_eval ? kWsTile : 0u);
+    P.warp_words = kWsHead + (P.grouped_tab ? kWsQueueWords : 0u) + areas * kWsTile;
     const size_t smem = 4ull * (2ull * P.chunk_words + (size_t)P.warp_words * kWsWarps +
                                 (P.grouped_tab ? 3ull * kWsGroupSlots : 0ull));
     if (smem > kWsMaxDynSmem) return GX_OK;

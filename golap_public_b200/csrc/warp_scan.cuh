@@ -13,49 +13,69 @@
 // start (chunk keep bits of the launch and their prefix counts, computed by
 // each CTA) no warp waits for another.  The 1024-row tiles of the surviving
 // chunks form a dense rank space; warp w of the grid takes tiles w, w + W,
-// w + 2W, ... (W warps), four at a time:
-//   * one decision round per four tiles: lane 8q + c reads column c's
-//     directory entry and side-index entries for tile q (a cascaded page's
-//     header and up to 8 runs too) and picks how the column is read --
-//     staged (raw rows or a 16-byte aligned LZ4 literal run: one bulk copy
-//     of the tile's rows into the warp's stage area), constant (a cascaded
-//     page or run that holds one value on the tile), or decoded by the warp
-//     into its buffer (LZ4 ranges with matches: groups of lanes per
-//     segment; other cascaded pages: run windows of 32 runs, one per lane);
-//     the round's staged ranges are bulk-prefetched into L2 and the next
-//     round's directory lines prefetched;
-//   * per tile: the bulk copies on the warp's mbarrier, the decodes, then the
-//     plan's steps over row groups of 128 rows (4 consecutive rows per lane,
-//     one 16-byte shared load per column).  Plans of the SSB shapes run a
-//     compile-time evaluator selected by their signature (all values of a
-//     row group in registers, steps over a constant column decided once per
-//     tile); other plans a run-time step-major evaluator.
-// Scalar sums stay in registers; grouped sums go to the CTA's group table in
-// shared memory (keys that find no slot go to the global table), flushed when
-// the CTA is done.  Join-table reads carry an L2 evict-last policy and the
-// streamed column bytes an evict-first one, so that the tables stay in L2
-// while the fact columns pass through it.
+// w + 2W, ... (W warps), and the tiles of the last, incomplete round are cut
+// into 256- or 512-row parts when there are warps to spare (so a pruned scan
+// of a few hundred tiles uses the whole chip, and a long one ends level).
+// Tiles are decided eight at a time (four for plans of more than 4 columns,
+// steps or predicates):
+//   * one decision round: lane (q << cl) + c reads column c's directory entry
+//     and side-index entries for tile q (a cascaded page's header and up to 8
+//     runs too) and writes to the warp's records in shared memory how the
+//     column is read -- direct (raw rows or a 16-byte aligned LZ4 literal run:
+//     the evaluator loads the rows from HBM itself), from the page's own bytes
+//     (bit-packed values, two runs, a few runs), constant (one value on the
+//     tile), or decoded by the warp into its buffer (LZ4 ranges with matches:
+//     groups of lanes per segment; other cascaded pages: run windows of 32
+//     runs, one per lane).  The next round's directory lines are prefetched,
+//     and the round's steps over constant columns decided, all in one chain of
+//     loads;
+//   * per tile: the decodes, then the plan's other steps over row groups of
+//     128 rows (4 consecutive rows per lane, one 16-byte load per column).
+//     Plans of the SSB shapes run a compile-time evaluator selected by their
+//     signature (all values of its row groups loaded before any is used);
+//     other plans the same evaluator with its steps read at run time.
+// Scalar sums stay in registers; grouped rows are collected per warp and
+// added, 32 at a time, to the CTA's group table in shared memory (keys that
+// find no slot go to the global table), flushed when the CTA is done.
+// Join-table reads carry an L2 evict-last policy, so that the tables stay in
+// L2 while the fact columns pass through it.
+//
+// What bounds it, and why it is built this way (B200, 148 SMs): a Q1 scan of
+// 60M rows has to read 747 MB, 114 us at the measured copy rate, and a loop
+// that only reads three columns in this tile pattern reaches 6.4 TB/s with 24
+// warps per SM and two row groups of loads in flight per warp.  Staging tiles
+// in shared memory held the kernel at 12 warps, waiting for its own copies:
+// 180 us; rows read in place, decisions in shared memory instead of registers,
+// row masks as predicates (1,400 -> 900 instructions per tile): 132 us.  The
+// star joins are bound by random table reads; there one row group per warp,
+// chains walked for all of a lane's rows together and dense group-table adds
+// took the 200M-row join from 6.3 to 2.2 ms, the four-join profit query over
+// 24M rows from 1.65 ms to 0.56 ms.  All-cascaded Q1 over 16M rows, values
+// unpacked in registers instead of through a decode buffer: 628 -> 205 us.
 
 constexpr uint32_t kWsLog2 = 10;
 constexpr uint32_t kWsTile = 1u << kWsLog2;    // rows of one warp tile
 constexpr uint32_t kWsNT = 128;                // threads per CTA (4 independent warps)
 constexpr uint32_t kWsWarps = kWsNT / 32;
 constexpr uint32_t kWsBatch = 128;             // rows of one row group (4 per lane)
-constexpr uint32_t kWsGroups = kWsTile / kWsBatch;  // row groups of a tile (4 keep bits each)
-constexpr uint32_t kWsEvalGroups = 2;               // row groups a scalar compile-time evaluator runs at once
+constexpr uint32_t kWsGroups = kWsTile / kWsBatch;  // row groups of a tile
+constexpr uint32_t kWsEvalGroups = 2;               // row groups an evaluator runs at once at most
+constexpr uint32_t kWsPartRows = kWsBatch * kWsEvalGroups;  // smallest part of a tile a warp takes
+constexpr uint32_t kWsMaxParts = kWsTile / kWsPartRows;
 static_assert(kWsGroups % kWsEvalGroups == 0, "the evaluator's row-group batches cover the tile");
-static_assert(kWsGroups * 4 <= 32, "the keep bits of a tile fit one word");
 constexpr uint32_t kWsMaxCols = kPipeMaxCols;
 constexpr uint32_t kWsGroupLog2 = 9;           // the CTA's group table: 512 slots
 constexpr uint32_t kWsGroupSlots = 1u << kWsGroupLog2;
-constexpr uint32_t kWsGroupProbes = 16;
 constexpr uint32_t kWsNone = 0xFFFFFFFFu;
 constexpr uint32_t kWsMaxDynSmem = 220u << 10;  // dynamic shared memory of one CTA at most
 constexpr uint32_t kWsMaxChunkWords = 1024;     // chunk keep bits of one launch: 32768 chunks
-// per-warp words before the stage: 8 constant slots (32 words), the mbarrier
-// (2 + 2 padding), the dense join tables' {base, span} headers per step (16)
-constexpr uint32_t kWsHead = 52;
-static_assert(4 * kWsMaxCols + 4 + 2 * GX_MAX_STEPS <= kWsHead && kWsHead % 4 == 0, "the warp head holds its parts");
+// per-warp words before the decode buffers: 32 column records of 8 words, 8
+// tile records of 8 words, the dense join tables' {base, span} headers per
+// step (16), the constant steps' group-key digits (32), the rows scanned (2,
+// and 2 of padding)
+constexpr uint32_t kWsHead = 32 * 8 + 8 * 8 + 2 * GX_MAX_STEPS + 32 + 4;
+constexpr uint32_t kWsQueueWords = (kWsBatch + 32) * 3;  // grouped plans: the warp's WsQueue, before its decode buffers
+static_assert(kWsHead % 4 == 0, "decode buffers start 16-byte aligned");
 static_assert(kWsTile <= kCascPageRows && kCascPageRows % kWsTile == 0, "a warp tile lies in one cascaded page");
 
 struct WsParams {
@@ -63,11 +83,14 @@ struct WsParams {
     gx_dcol cols[kWsMaxCols];
     uint32_t n_cols;
     uint32_t blocks_per_chunk, rows_per_chunk, rows_per_block, tiles_per_block;
+    // division by the tiles per chunk and per block, for numerators below 2^31
+    uint32_t pc_mul, pc_shift, tpb_mul, tpb_shift;
+    uint32_t col_log2;              // decision rounds: 4 lanes per tile (at most 4 columns, steps, predicates) or 8
+    uint32_t parts;                 // 1: tiles of the last round may be cut (no column needs an LZ4 decode)
     uint64_t n_rows;                // rows of the table
     uint32_t chunk_lo, chunk_hi;    // chunks [chunk_lo, chunk_hi) are scanned
-    uint32_t stage_of[kWsMaxCols];  // stage area column c is copied into (raw / aligned-literal LZ4), or kWsNone
     uint32_t buf_of[kWsMaxCols];    // decode buffer of column c (cascaded / LZ4 with matches), or kWsNone
-    uint32_t n_areas;               // stage areas + decode buffers per warp (kWsTile words each)
+    uint32_t n_areas;               // decode buffers per warp (kWsTile words each)
     uint32_t warp_words;            // shared memory words per warp
     uint32_t chunk_words;           // words of the chunk keep bitmap (and of its prefix counts)
     uint32_t grouped_tab;           // 1: the warp has a group table
@@ -75,14 +98,17 @@ struct WsParams {
 };
 
 // Column read modes of one tile.
-// kWmRuns2: a cascaded tile covered by two runs (value cval on tile rows
-// [0, aux0), value aux1 from there), written out without the page decoder.
-enum : uint32_t { kWmStage = 0, kWmConst = 1, kWmLz4 = 2, kWmCasc = 3, kWmBad = 4, kWmRuns2 = 5 };
-
-__device__ __forceinline__ uint64_t ws_shfl64(uint64_t v, uint32_t src) {
-    return ((uint64_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)(v >> 32), src) << 32) |
-           __shfl_sync(0xFFFFFFFFu, (uint32_t)v, src);
-}
+// kWmDirect: the tile's rows lie in memory as they are (raw, or inside one
+// 16-byte aligned LZ4 literal run) and the evaluator loads them itself.
+// Cascaded pages that the evaluator reads from their own bytes, without a
+// decode: kWmPack, bit-packed values without RLE or DELTA (four values of a
+// lane from up to five words); kWmRuns2, a tile of a few-run page covered by
+// two runs (value cval on tile rows [0, aux0), value aux1 from there);
+// kWmRuns, a tile of more runs of such a page.
+// kWmRows: in shared memory, after the warp's decode.
+enum : uint32_t {
+    kWmDirect = 0, kWmConst = 1, kWmLz4 = 2, kWmCasc = 3, kWmBad = 4, kWmRuns2 = 5, kWmRows = 6, kWmPack = 7, kWmRuns = 8
+};
 
 // Inclusive warp scan (wrapping uint32 sum).
 __device__ __forceinline__ uint32_t ws_scan(uint32_t x, uint32_t lane) {
@@ -92,15 +118,6 @@ __device__ __forceinline__ uint32_t ws_scan(uint32_t x, uint32_t lane) {
         if (lane >= (uint32_t)d) x += y;
     }
     return x;
-}
-
-// One bulk copy (no multicast) completing on m, its lines read under policy pol.
-__device__ __forceinline__ void ws_bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* m, uint64_t pol) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::
-            "r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(m)), "l"(pol)
-        : "memory");
 }
 
 // Rows [h0, h0 + n) of a cascaded page decoded by one warp into out[0..n),
@@ -220,23 +237,73 @@ __device__ __noinline__ int ws_lz4_rows(const uint8_t* blk, uint32_t blk_bytes, 
     return __any_sync(0xFFFFFFFFu, err != 0) ? kErrCorrupt : 0;
 }
 
-// Add of (gk, val) to the warp's group table; keys that find no slot within
-// kWsGroupProbes go to the global table.
-__device__ __forceinline__ void ws_group_add(uint32_t gk, int64_t val, uint32_t* tkey, unsigned long long* tsum,
-                                          int64_t* keys, int64_t* sums, uint32_t log2cap) {
+// Add of (key, val) to the CTA's group table in shared memory: sets of four
+// slots, the key's set and the next one; a key that finds no slot there goes
+// to the global table.  The sums are kept as 32-bit halves (a shared 64-bit
+// add is a compare-and-swap loop): the low half's old value tells the carry.
+__device__ __forceinline__ void ws_group_add(uint32_t gk, int64_t val, uint32_t* tkey, uint32_t* tlo, uint32_t* thi,
+                                             int64_t* keys, int64_t* sums, uint32_t log2cap) {
     if (gk != kEmptyGKey) {
-        uint32_t s = hash_key32((int32_t)gk, kWsGroupLog2);
-        for (uint32_t i = 0; i < kWsGroupProbes; ++i) {
-            uint32_t cur = ((volatile uint32_t*)tkey)[s];
-            if (cur == kEmptyGKey) cur = atomicCAS(&tkey[s], kEmptyGKey, gk);
-            if (cur == kEmptyGKey || cur == gk) {
-                atomicAdd(&tsum[s], (unsigned long long)val);
+        const uint32_t s0 = hash_key32((int32_t)gk, kWsGroupLog2) & ~3u;
+#pragma unroll 1
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t b = (s0 + 4 * i) & (kWsGroupSlots - 1);
+            uint32_t x[4];
+            asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+                         : "r"(smem_u32(tkey + b))
+                         : "memory");
+            uint32_t slot = kWsNone;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (x[j] == gk) slot = b + j;
+            if (slot == kWsNone) {
+                // not there yet: the first free slot of the set (a slot another
+                // thread takes meanwhile is passed over unless it took it for gk)
+#pragma unroll 1
+                for (uint32_t j = 0; j < 4 && slot == kWsNone; ++j) {
+                    if (x[j] != kEmptyGKey) continue;
+                    const uint32_t old = atomicCAS(&tkey[b + j], kEmptyGKey, gk);
+                    if (old == kEmptyGKey || old == gk) slot = b + j;
+                }
+            }
+            if (slot != kWsNone) {
+                const uint32_t lo = (uint32_t)(uint64_t)val;
+                const uint32_t old = atomicAdd(&tlo[slot], lo);
+                const uint32_t hi = (uint32_t)((uint64_t)val >> 32) + (old + lo < old ? 1u : 0u);
+                if (hi) atomicAdd(&thi[slot], hi);
                 return;
             }
-            s = (s + 1) & (kWsGroupSlots - 1);
         }
     }
     if (!group_add_global(keys, sums, log2cap, (int64_t)gk, val)) raise_error(kErrCapacity);
+}
+
+// The grouped rows of a warp on their way to the group table: few rows of a
+// row group survive a star join's probes, so they are collected in shared
+// memory until 32 of them fill the warp's lanes (room for the rows of a batch and a
+// rest of 31).
+constexpr uint32_t kWsQueue = kWsBatch + 32;
+struct WsQueue {
+    int64_t val[kWsQueue];
+    uint32_t key[kWsQueue];
+};
+
+// One row per lane (lanes with `on`).
+__device__ __noinline__ void ws_group_add_lanes(bool on, uint32_t gk, int64_t val, uint32_t* tkey, int64_t* keys,
+                                                int64_t* sums, uint32_t log2cap) {
+    if (on) ws_group_add(gk, val, tkey, tkey + kWsGroupSlots, tkey + 2 * kWsGroupSlots, keys, sums, log2cap);
+    __syncwarp();
+}
+
+// The queue's newest n rows (at most 32, qn of them after) into the table.
+__device__ __noinline__ void ws_queue_flush(const WsQueue* wq, uint32_t qn, uint32_t n, uint32_t* tkey, int64_t* keys,
+                                            int64_t* sums, uint32_t log2cap, uint32_t lane) {
+    __syncwarp();
+    if (lane < n)
+        ws_group_add(wq->key[qn + lane], wq->val[qn + lane], tkey, tkey + kWsGroupSlots, tkey + 2 * kWsGroupSlots,
+                     keys, sums, log2cap);
+    __syncwarp();
 }
 
 // Position of the k-th set bit of m (k < popc(m)).
@@ -255,48 +322,80 @@ __device__ __forceinline__ uint32_t ws_select(uint32_t m, uint32_t k) {
 }
 
 // One row tile: block slot, first row in the block, rows, block rows, and
-// the rows [a, b) of the tile inside the query's row slice.
-struct WsTile {
+// the rows [a, b) of the tile that the warp evaluates (all of them, or the
+// part of a tile cut for the last round).
+struct __align__(16) WsTile {
     uint32_t slot, r0, n, rows, a, b;
+    uint32_t steps;  // bit s: step s is over a constant column; kWsDead, kWsBroadcast
+    uint32_t pad;
 };
+constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
+constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a probe's constant or two-run one
+static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
 
 // How one column of one tile is read.
-struct WsCol {
+struct __align__(16) WsCol {
+    const uint8_t* src;   // direct, kWmRows: the rows; LZ4: the block; cascaded: the page; kWmPack: its values
     uint32_t mode;        // kWm*
-    const uint8_t* src;   // stage: the rows; LZ4: the block; cascaded: the page
-    uint32_t aux0, aux1;  // LZ4: [lo, hi) in the block; cascaded: page bytes, page rows
-    uint32_t bytes;       // stage: bytes copied; LZ4: the block's compressed bytes
-    int32_t cval;         // kWmConst: the value
+    int32_t cval;         // kWmConst: the value; kWmRuns2: the first run's; kWmPack: the frame of reference
+    uint32_t aux0, aux1;  // LZ4: [lo, hi) in the block; cascaded: page bytes, page rows; kWmRuns2: the first
+                          // run's end, the second's value; kWmPack: bits per value
+    uint32_t bytes;       // LZ4: the block's compressed bytes; kWmPack, kWmRuns: the tile's first row in the page
+    uint32_t pad;
+};
+static_assert(sizeof(WsCol) == 32, "column records of 8 words");
+
+// n / d for n < 2^31, d's multiplier and shift computed by the host.
+__device__ __forceinline__ uint32_t ws_div(uint32_t n, uint32_t mul, uint32_t shift) {
+    return (uint32_t)(((uint64_t)n * mul) >> shift);
+}
+
+// The launch's work, the same for every warp: `first` is the first surviving
+// chunk when they are neighbours (a range predicate on a sorted column, no
+// pruning), else kWsNone and a chunk is found by its rank in the keep bits.
+// t_end tiles go to W warps: `full` rounds of W whole tiles, then the tiles
+// left over, cut into 1 << parts_log2 parts, one per warp.
+struct WsWork {
+    uint32_t first, t_end, W, full, rounds, parts_log2;
 };
 
-// Rank-space tile t (t-th tile of the surviving chunks, chunk-major) ->
-// its tile; false when t is past the end or the tile has no rows of the
-// query's slice.
+// Tile number t of the surviving chunks (chunk-major) -> its tile, whole;
+// false when t is past the end or the chunk has no such rows.
 __device__ __forceinline__ bool ws_locate(const WsParams& P, const uint32_t* s_kbits, const uint32_t* s_kpre,
-                                          uint32_t t, uint32_t t_end, WsTile& T) {
-    if (t >= t_end) return false;
+                                          const WsWork& R, uint32_t t, WsTile& T) {
+    if (t >= R.t_end) return false;
     const uint32_t tpb = P.tiles_per_block, bpc = P.blocks_per_chunk;
-    const uint32_t PC = bpc * tpb;  // the launch keeps tile indices below 2^31
-    const uint32_t k = t / PC, loc = t - k * PC;
-    uint32_t lo = 0, hi = P.chunk_words - 1;  // the bitmap word holding the k-th surviving chunk
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (s_kpre[mid] <= k) lo = mid; else hi = mid - 1;
+    const uint32_t k = ws_div(t, P.pc_mul, P.pc_shift), loc = t - k * (bpc * tpb);
+    uint32_t chunk = R.first + k;
+    if (R.first == kWsNone) {
+        uint32_t lo = 0, hi = P.chunk_words - 1;  // the bitmap word holding the k-th surviving chunk
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1) >> 1;
+            if (s_kpre[mid] <= k) lo = mid; else hi = mid - 1;
+        }
+        chunk = P.chunk_lo + lo * 32 + ws_select(s_kbits[lo], k - s_kpre[lo]);
     }
-    const uint32_t chunk = P.chunk_lo + lo * 32 + ws_select(s_kbits[lo], k - s_kpre[lo]);
-    const uint32_t jb = loc / tpb, tile = loc % tpb;
-    const uint64_t c_r0 = (uint64_t)chunk * P.rows_per_chunk;
-    const uint64_t c_rows = min((uint64_t)P.rows_per_chunk, P.n_rows - c_r0);
+    const uint32_t jb = ws_div(loc, P.tpb_mul, P.tpb_shift), tile = loc - jb * tpb;
+    const uint64_t c_rows = min((uint64_t)P.rows_per_chunk, P.n_rows - (uint64_t)chunk * P.rows_per_chunk);
     const uint64_t jrow = (uint64_t)jb * P.rows_per_block;
     T.rows = jrow < c_rows ? (uint32_t)min((uint64_t)P.rows_per_block, c_rows - jrow) : 0u;
     T.r0 = tile * kWsTile;
     T.slot = chunk * bpc + jb;
     if (T.r0 >= T.rows) return false;
     T.n = min(kWsTile, T.rows - T.r0);
-    const uint64_t g0 = c_r0 + jrow + T.r0;
-    const ShQuery& Q = P.q;
-    T.a = Q.row_lo > g0 ? (uint32_t)min((uint64_t)T.n, Q.row_lo - g0) : 0u;
-    T.b = Q.row_hi > g0 ? (uint32_t)min((uint64_t)T.n, Q.row_hi - g0) : 0u;
+    T.a = 0;
+    T.b = T.n;
+    return true;
+}
+
+// Warp w's piece of round r.
+__device__ __forceinline__ bool ws_piece(const WsParams& P, const uint32_t* s_kbits, const uint32_t* s_kpre,
+                                         const WsWork& R, uint32_t w, uint32_t r, WsTile& T) {
+    if (r < R.full) return ws_locate(P, s_kbits, s_kpre, R, r * R.W + w, T);
+    if (r > R.full || !ws_locate(P, s_kbits, s_kpre, R, r * R.W + (w >> R.parts_log2), T)) return false;
+    const uint32_t part = kWsTile >> R.parts_log2, p0 = (w & ((1u << R.parts_log2) - 1u)) * part;
+    T.a = p0;
+    T.b = min(T.n, p0 + part);
     return T.a < T.b;
 }
 
@@ -316,10 +415,9 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
         d_rows == rows && d_off <= col.payload_bytes && (uint64_t)d_bytes + 32 <= col.payload_bytes - d_off;
     const uint8_t* blk = col.payload + d_off;
     if (col.codec == GX_CODEC_NONE) {
-        if (dir_ok && d_bytes == rows * 4 && (d_off & 15u) == 0 && P.stage_of[c] != kWsNone) {
-            C.mode = kWmStage;
+        if (dir_ok && d_bytes == rows * 4 && (d_off & 15u) == 0) {
+            C.mode = kWmDirect;
             C.src = blk + 4ull * r0;
-            C.bytes = (4 * n + 15u) & ~15u;
         }
     } else if (col.codec == GX_CODEC_LZ4) {
         const uint32_t sr = 1u << col.seg_shift;
@@ -331,10 +429,9 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
             const uint32_t hi = j0 + nseg < col.S ? e2 : d_bytes;
             if (dir_ok && e0 <= hi && hi <= d_bytes) {
                 const bool lit = (e1 & 16u) && (e1 >> 5) >= 4 * n && hi - e0 == 4 * n;
-                if (lit && ((d_off + e0) & 15u) == 0 && P.stage_of[c] != kWsNone) {
-                    C.mode = kWmStage;
+                if (lit && ((d_off + e0) & 15u) == 0) {
+                    C.mode = kWmDirect;
                     C.src = blk + e0;
-                    C.bytes = (4 * n + 15u) & ~15u;
                 } else if (P.buf_of[c] != kWsNone) {
                     C.mode = kWmLz4;
                     C.src = blk;
@@ -346,12 +443,12 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
         }
     } else if (col.codec == GX_CODEC_CASCADED) {
         const uint32_t page = r0 >> kCascPageLog2;
-        if (page < col.S && P.buf_of[c] != kWsNone) {
+        if (page < col.S) {
             const uint32_t* e = col.seg + (size_t)2 * col.S * slot + 2 * page;
             const uint32_t po = __ldg(e), pb = __ldg(e + 1);
             if (dir_ok && (d_off & 15u) == 0 && (po & 15u) == 0 && (uint64_t)po + pb <= d_bytes && pb >= 32) {
                 const uint8_t* pg = blk + po;
-                C.mode = kWmCasc;
+                if (P.buf_of[c] != kWsNone) C.mode = kWmCasc;
                 C.src = pg;
                 C.aux0 = pb;
                 C.aux1 = min(kCascPageRows, rows - page * kCascPageRows);
@@ -363,7 +460,13 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
                     if (!rle && h.val_bits == 0 && (!delta || h.val_base == 0)) {
                         C.mode = kWmConst;
                         C.cval = delta ? h.first : h.val_base;
-                    } else if (rle && h.n_runs <= 8) {
+                    } else if (!rle && !delta) {
+                        C.mode = kWmPack;
+                        C.src = pg + h.vals_off;
+                        C.cval = h.val_base;
+                        C.aux0 = h.val_bits;
+                        C.bytes = r0 & (kCascPageRows - 1u);
+                    } else if (rle && h.n_runs <= kCascFewRuns) {
                         // a few runs (sorted columns): the run holding the tile's first
                         // row, and whether it also holds the last
                         const uint32_t* vw = (const uint32_t*)(pg + h.vals_off);
@@ -397,6 +500,13 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
                                 break;
                             }
                         }
+                        if (C.mode != kWmConst && C.mode != kWmRuns2) {
+                            // more runs on the tile: read run by run, if they add up to the page
+                            uint32_t sum = 0;
+                            for (uint32_t k = 0; k < h.n_runs; ++k) sum += unpack_bits(lw, k, h.len_bits) + h.len_base;
+                            C.mode = sum == C.aux1 ? kWmRuns : kWmBad;
+                            C.bytes = h0;
+                        }
                     }
                 }
             }
@@ -405,226 +515,108 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
     return C;
 }
 
-// Decisions for the four tiles t0 + q*W (q = 0..3) at once: lane 8q + c
-// decides column c of tile q (and checks prune predicate c's zone map), so
-// the four tiles cost one round of dependent loads.  Returns the mask of
-// the tiles to scan; every lane of group q holds tile q in T.
-__device__ __forceinline__ uint32_t ws_decide(const WsParams& P, const gx_dcol* s_cols, const uint32_t* s_kbits,
-                                              const uint32_t* s_kpre, uint32_t t0, uint32_t W, uint32_t t_end,
-                                              uint32_t lane, WsTile& T, WsCol& C) {
+// Decisions for warp w's pieces of the 32 >> cl rounds from r0 on at once (cl:
+// WsParams::col_log2): lane (q << cl) + c decides column c of round r0 + q
+// (and checks prune predicate c's zone map), so that eight tiles of a narrow
+// plan or four of a wide one cost one chain of dependent loads, and the
+// directory and side-index lines of the rounds after them are prefetched into
+// L2.  The records go to tiles[q] and cols[(q << cl) + c]; returns the mask of
+// the tiles to scan.  Out of line: its registers are not the evaluator's.
+__device__ __noinline__ uint32_t ws_decide(const WsParams& P, const gx_dcol* s_cols, const uint32_t* s_kbits,
+                                           const uint32_t* s_kpre, const WsWork& R, uint32_t w, uint32_t r0,
+                                           uint32_t lane, WsTile* tiles, WsCol* cols) {
     const ShQuery& Q = P.q;
-    const uint32_t q = lane >> 3, c = lane & 7;
-    const bool ok = ws_locate(P, s_kbits, s_kpre, t0 + q * W, t_end, T);
+    const uint32_t cl = P.col_log2, q = lane >> cl, c = lane & ((1u << cl) - 1u), nq = 32u >> cl;
+    WsTile T;
+    const bool ok = ws_piece(P, s_kbits, s_kpre, R, w, r0 + q, T);
     bool zfail = false;
     if (ok && c < Q.n_prune) {
         const PrunePred& pr = Q.prune[c];
         if (pr.bmins) zfail = !(pr.lo <= __ldg(pr.bmaxs + T.slot) && pr.hi >= __ldg(pr.bmins + T.slot));
     }
-    C.mode = kWmBad;
-    if (ok && c < P.n_cols) C = ws_column(P, s_cols[c], c, T);
+    if (ok && c < P.n_cols) {
+        const WsCol C = ws_column(P, s_cols[c], c, T);
+        cols[lane] = C;
+        if (C.mode == kWmPack) {  // the tile's packed values to L2 (inside the payload's slack)
+            const uintptr_t p0 = ((uintptr_t)C.src + ((uint64_t)(C.bytes + T.a) * C.aux0) / 8) & ~(uintptr_t)15;
+            const uintptr_t p1 = ((uintptr_t)C.src + ((uint64_t)(C.bytes + T.b) * C.aux0) / 8 + 15) & ~(uintptr_t)15;
+            if (p1 > p0)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p0), "r"((uint32_t)(p1 - p0))
+                             : "memory");
+        }
+    }
+    if (ok && c == 0) tiles[q] = T;
     const uint32_t oks = __ballot_sync(0xFFFFFFFFu, ok), fails = __ballot_sync(0xFFFFFFFFu, zfail);
     uint32_t vm = 0;
-#pragma unroll
-    for (uint32_t g = 0; g < 4; ++g)
-        if (((oks >> (8 * g)) & 1u) && ((fails >> (8 * g)) & 0xFFu) == 0) vm |= 1u << g;
+    for (uint32_t g = 0; g < nq; ++g)
+        if (((oks >> (g << cl)) & 1u) && ((fails >> (g << cl)) & ((1u << (1u << cl)) - 1u)) == 0) vm |= 1u << g;
+    if (c < P.n_cols && r0 + nq + q < R.rounds && ws_piece(P, s_kbits, s_kpre, R, w, r0 + nq + q, T)) {
+        const gx_dcol& col = s_cols[c];
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(col.blocks + T.slot));
+        if (col.codec != GX_CODEC_NONE)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(col.seg + (size_t)2 * col.S * T.slot +
+                                                          2 * (T.r0 >> col.seg_shift)));
+    }
+    __syncwarp();
     return vm;
 }
 
-// L2 prefetch of the directory and side-index lines of the four tiles
-// t0 + q*W (lane 8q + c: column c), so that their decisions read L2.
-__device__ __forceinline__ void ws_prefetch_meta(const WsParams& P, const gx_dcol* s_cols, const uint32_t* s_kbits,
-                                                 const uint32_t* s_kpre, uint32_t t0, uint32_t W, uint32_t t_end,
-                                                 uint32_t lane) {
-    const uint32_t q = lane >> 3, c = lane & 7;
-    WsTile T;
-    if (c >= P.n_cols || !ws_locate(P, s_kbits, s_kpre, t0 + q * W, t_end, T)) return;
-    const gx_dcol& col = s_cols[c];
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(col.blocks + T.slot));
-    if (col.codec == GX_CODEC_LZ4)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(col.seg + (size_t)2 * col.S * T.slot + 2 * (T.r0 >> col.seg_shift)));
-    else if (col.codec == GX_CODEC_CASCADED)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(col.seg + (size_t)2 * col.S * T.slot + 2 * (T.r0 >> kCascPageLog2)));
+// One key in a join table: dense tables through their cached header.
+__device__ __forceinline__ bool ws_probe1(const ShStep& st, uint64_t hdr, int32_t v, int32_t* p, uint64_t pol_keep) {
+    if (st.ht_layout != GX_HT_DENSE) return ht_probe_any(st.ht, st.ht_log2, st.ht_layout, v, p);
+    const uint32_t u = (uint32_t)v - (uint32_t)hdr;
+    if (v == kEmptyKey || u >= (uint32_t)(hdr >> 32)) return false;
+    const unsigned long long e = ws_ld_slot((const unsigned long long*)st.ht + 1 + u, pol_keep);
+    if ((int32_t)(uint32_t)e != v) return false;
+    *p = (int32_t)(uint32_t)(e >> 32);
+    return true;
 }
 
-__device__ __forceinline__ void ws_bulk_prefetch_l2(const void* src, uint32_t bytes, uint64_t pol) {
-    asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(src), "r"(bytes), "l"(pol)
-                 : "memory");
-}
-
-// A step over a column that holds one value v on the whole tile: decided
-// once.  Returns true when the tile's rows are all dropped; else multiplies
-// in the group-key digit of every kept row.
-__device__ __forceinline__ bool ws_step_const(const ShStep& stp, int32_t v, uint32_t keep, uint32_t* gkb, bool grouped,
-                                           uint32_t lane) {
-    const uint32_t flags = stp.flags, dcard = stp.digit_card;
-    bool f = !(flags & GX_STEP_FILTER) || (v >= stp.lo && v <= stp.hi);
-    int32_t pp = v;
-    if (f && (flags & GX_STEP_PROBE)) f = ht_probe_any(stp.ht, stp.ht_log2, stp.ht_layout, v, &pp);
-    if (!f) return true;
-    if (dcard && grouped) {
-        const uint32_t dgt = (uint32_t)(pp - stp.digit_base);
-        if (dgt >= dcard) {
-            if (lane == 0) raise_error(kErrInvalid);
-            return true;
-        }
-#pragma unroll 1
-        for (uint32_t j = 0; j < kWsGroups; ++j) {
-            if (!((keep >> (4 * j)) & 15u)) continue;
-            uint4* g = (uint4*)(gkb + 128 * j + 4 * lane);
-            uint4 x = *g;
-            x.x = x.x * dcard + dgt;
-            x.y = x.y * dcard + dgt;
-            x.z = x.z * dcard + dgt;
-            x.w = x.w * dcard + dgt;
-            *g = x;
-        }
-    }
-    return false;
-}
-
-// A filter / probe / digit step over the tile's rows of a column at `col`
-// (shared memory, kWsTile rows).  Probes issue the first-slot reads of a
-// row group's distinct keys together and reuse the lane's last result for a
-// repeated key.  Returns the new keep bits.
-__device__ __forceinline__ uint32_t ws_step_rows(const ShStep& stp, const uint8_t* col, uint32_t keep, uint32_t* gkb,
-                                              bool grouped, uint64_t pol_keep, uint32_t lane) {
-    const uint32_t flags = stp.flags, dcard = stp.digit_card;
-    const int32_t lo = stp.lo, hi = stp.hi, dbase = stp.digit_base;
-    const bool filt = (flags & GX_STEP_FILTER) != 0, probe = (flags & GX_STEP_PROBE) != 0;
-    const uint64_t* const ht = stp.ht;
-    const uint32_t htlog = stp.ht_log2, htlay = stp.ht_layout;
-    const bool dense = htlay == GX_HT_DENSE, bucket = htlay == GX_HT_BUCKET;
-    uint32_t hbase = 0, hspan = 0;
-    if (probe && dense) {
-        const uint64_t hdr = __ldg((const unsigned long long*)ht);
-        hbase = (uint32_t)hdr;
-        hspan = (uint32_t)(hdr >> 32);
-    }
-    int32_t mv = 0, mp = 0;  // the lane's last probed key and its result
-    bool mhave = false, mf = false;
-#pragma unroll 1
-    for (uint32_t j = 0; j < kWsGroups; ++j) {
-        uint32_t kk = (keep >> (4 * j)) & 15u;
-        if (!kk) continue;
-        const uint4 w4 = *(const uint4*)(col + (128 * j + 4 * lane) * 4);
-        const int32_t v[4] = {(int32_t)w4.x, (int32_t)w4.y, (int32_t)w4.z, (int32_t)w4.w};
-        if (filt) {
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i)
-                if (!(v[i] >= lo && v[i] <= hi)) kk &= ~(1u << i);
-        }
-        int32_t pp[4] = {v[0], v[1], v[2], v[3]};
-        if (probe && kk) {
-            uint64_t ee[4];
-            uint32_t rd = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                const bool again =
-                    (i > 0 && v[i] == v[i - 1] && ((kk >> (i - 1)) & 1u)) || (mhave && v[i] == mv);
-                const uint32_t u = (uint32_t)v[i] - hbase;
-                const bool r = ((kk >> i) & 1u) && !again && !bucket && v[i] != kEmptyKey && (!dense || u < hspan);
-                const unsigned long long* sl = (const unsigned long long*)ht + (dense ? 1 + u : hash_key32(v[i], htlog));
-                ee[i] = r ? ws_ld_slot(sl, pol_keep) : (unsigned long long)kEmptySlot;
-                rd |= r ? 1u << i : 0u;
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                if (!((kk >> i) & 1u)) continue;
-                bool f;
-                int32_t p = v[i];
-                if (mhave && v[i] == mv) {
-                    f = mf;
-                    p = mp;
-                } else if ((rd >> i) & 1u) {
-                    const int32_t ek = (int32_t)(uint32_t)ee[i];
-                    if (ek == v[i]) {
-                        f = true;
-                        p = (int32_t)(uint32_t)(ee[i] >> 32);
-                    } else if (dense || ek == kEmptyKey) {
-                        f = false;
-                    } else {
-                        f = sh_probe(ht, htlog, htlay, v[i], &p);
-                    }
-                } else {
-                    // bucket tables, keys the memo held when the reads were issued,
-                    // the reserved key, keys outside a dense range
-                    f = sh_probe(ht, htlog, htlay, v[i], &p);
-                }
-                mhave = true;
-                mv = v[i];
-                mf = f;
-                mp = p;
-                pp[i] = p;
-                if (!f) kk &= ~(1u << i);
-            }
-        }
-        if (dcard && grouped && kk) {
-            uint4* g = (uint4*)(gkb + 128 * j + 4 * lane);
-            const uint4 x = *g;
-            uint32_t xg[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                if (!((kk >> i) & 1u)) continue;
-                const uint32_t dgt = (uint32_t)(pp[i] - dbase);
-                if (dgt >= dcard) {
-                    raise_error(kErrInvalid);
-                    kk &= ~(1u << i);
-                } else {
-                    xg[i] = xg[i] * dcard + dgt;
-                }
-            }
-            *g = make_uint4(xg[0], xg[1], xg[2], xg[3]);
-        }
-        keep = (keep & ~(15u << (4 * j))) | (kk << (4 * j));
-    }
-    return keep;
-}
-
-// The aggregate over the kept rows of the tile: the value column at `col`
-// (mask 0: one value), the carried column at `ccol`.  Returns the scalar
-// part; grouped sums go to the warp's group table.
-__device__ __forceinline__ int64_t ws_aggregate(uint32_t agg, bool grouped, bool carried, const uint8_t* col, uint32_t msk,
-                                             const uint8_t* ccol, uint32_t cmask, uint32_t keep, const uint32_t* gkb,
-                                             uint32_t* tkey, unsigned long long* tsum, int64_t* g_keys,
-                                             int64_t* g_sums, uint32_t g_log2, uint32_t lane) {
-    if (!grouped && agg == GX_AGG_COUNT) return __popc(keep);
-    if (!grouped && agg == GX_AGG_SUM && msk == 0) return (int64_t)__popc(keep) * *(const int32_t*)col;
-    int64_t acc = 0;
-#pragma unroll 1
-    for (uint32_t j = 0; j < kWsGroups; ++j) {
-        const uint32_t kk = (keep >> (4 * j)) & 15u;
-        if (!kk) continue;
-        const uint32_t ro = (128 * j + 4 * lane) * 4;
-        const uint4 w4 = *(const uint4*)(col + (ro & msk));
-        const uint4 cw = carried ? *(const uint4*)(ccol + (ro & cmask)) : make_uint4(0, 0, 0, 0);
-        const int32_t v[4] = {(int32_t)w4.x, (int32_t)w4.y, (int32_t)w4.z, (int32_t)w4.w};
-        const int32_t cv[4] = {(int32_t)cw.x, (int32_t)cw.y, (int32_t)cw.z, (int32_t)cw.w};
-        if (!grouped) {
-            if (agg == GX_AGG_SUM_PRODUCT) {
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) acc += ((kk >> i) & 1u) ? (int64_t)v[i] * cv[i] : 0;
-            } else if (agg == GX_AGG_SUM_DIFF) {
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) acc += ((kk >> i) & 1u) ? (int64_t)v[i] - cv[i] : 0;
-            } else {
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) acc += ((kk >> i) & 1u) ? (int64_t)v[i] : 0;
-            }
-        } else {
-            const uint4 gw = *(const uint4*)(gkb + 128 * j + 4 * lane);
-            const uint32_t g[4] = {gw.x, gw.y, gw.z, gw.w};
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                if (!((kk >> i) & 1u)) continue;
-                const int64_t val = agg == GX_AGG_SUM_PRODUCT ? (int64_t)v[i] * cv[i]
-                                    : agg == GX_AGG_SUM_DIFF  ? (int64_t)v[i] - cv[i]
-                                    : agg == GX_AGG_COUNT      ? 1
-                                                               : (int64_t)v[i];
-                ws_group_add(g[i], val, tkey, tsum, g_keys, g_sums, g_log2);
+// The steps over columns that hold one value on their tile, decided once per
+// tile and for all tiles of the round together (their probes are one chain of
+// loads): lane (q << cl) + s decides step s of tile q, leaves its group-key
+// digit in sdig[lane] (kWsNone: out of range) and tiles[q].steps says which
+// steps are constant and whether one of them drops every row.
+template <uint32_t SIG>
+__device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, WsTile* tiles, const WsCol* cols,
+                                               const uint64_t* whdr, uint32_t* sdig, uint64_t pol_keep,
+                                               uint32_t lane) {
+    const ShQuery& Q = P.q;
+    const uint32_t cl = P.col_log2, q = lane >> cl, s = lane & ((1u << cl) - 1u);
+    bool isc = false, ok = true, bad = false, mixed = false;
+    if (((vm >> q) & 1u) && s < Q.n_steps) {
+        const ShStep& st = Q.steps[s];
+        const WsCol& c = cols[(q << cl) + st.col];
+        isc = c.mode == kWmConst;
+        mixed = c.mode != kWmDirect && !((isc || c.mode == kWmRuns2) && (st.flags & GX_STEP_PROBE));
+        if (isc) {
+            const int32_t v = c.cval;
+            int32_t pp = v;
+            if (st.flags & GX_STEP_FILTER) ok = v >= st.lo && v <= st.hi;
+            if (ok && (st.flags & GX_STEP_PROBE)) ok = ws_probe1(st, whdr[s], v, &pp, pol_keep);
+            if (ok && st.digit_card) {
+                const uint32_t dgt = (uint32_t)(pp - st.digit_base);
+                bad = dgt >= st.digit_card;
+                sdig[lane] = bad ? kWsNone : dgt;
             }
         }
     }
-    return acc;
+    const uint32_t m0 = (1u << (1u << cl)) - 1u, sh = q << cl;
+    const uint32_t cst = (__ballot_sync(0xFFFFFFFFu, isc) >> sh) & m0;
+    const uint32_t fails = (__ballot_sync(0xFFFFFFFFu, isc && !ok) >> sh) & m0;
+    const uint32_t bads = (__ballot_sync(0xFFFFFFFFu, bad) >> sh) & m0;
+    const uint32_t mixes = (__ballot_sync(0xFFFFFFFFu, mixed) >> sh) & m0;
+    if (s == 0 && ((vm >> q) & 1u)) {
+        uint32_t f = cst | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
+        if (SIG != 0 && bads) {
+            // a digit out of range is an error unless a constant step before it drops
+            // the rows; the run-time evaluator raises it only for rows alive at the step
+            if ((fails & ((1u << (__ffs(bads) - 1)) - 1u)) == 0) raise_error(kErrInvalid);
+            f |= kWsDead;
+        }
+        tiles[q].steps = f;
+    }
+    __syncwarp();
 }
 
 // ---- plan signatures: compile-time evaluators for the known query shapes
@@ -646,263 +638,423 @@ constexpr uint32_t kSigQ2 = ws_sig(4, GX_AGG_SUM, true, kWkP | kWkD, kWkP, kWkP 
 // pipeline_q4: customer (nation digit), supplier, date (year digit), part probes, supplycost carried, profit grouped
 constexpr uint32_t kSigQ4 = ws_sig(6, GX_AGG_SUM_DIFF, true, kWkP | kWkD, kWkP, kWkP | kWkD, kWkP, kWkC, 0);
 
-// The tile's rows evaluated through all steps of a compile-time signature,
-// one 128-row group at a time: every column's 4 values of the lane are
-// loaded first, then the steps run on registers (carried values and group
-// keys included).  Steps over a column that holds one value on the tile
-// (other than the last) are decided once for the tile.  Returns the scalar
-// part; grouped sums go to the warp's group table.
-template <uint32_t SIG>
-__device__ __forceinline__ int64_t ws_eval_sig(const ShQuery& Q, const uint8_t* sbase, const uint32_t* off,
-                                               const uint32_t* msk, uint32_t keep, uint32_t* tkey,
-                                               unsigned long long* tsum, uint64_t pol_keep, const uint64_t* s_hdr,
-                                               uint32_t lane) {
-    constexpr uint32_t NS = SIG & 7, AGG = (SIG >> 3) & 7;
-    constexpr bool GR = ((SIG >> 6) & 1) != 0;
-    int64_t acc = 0;
-    uint32_t cd[NS];  // constant steps: the group-key digit
-    int32_t cv[NS];   // constant steps: the value
+// A join-table probe of R rows per lane (R = 4 per row group): rows whose bit
+// in m is set and whose key is found keep their bit, with their payload in
+// pay.  All rows' reads of a round are in flight together, a round reads two
+// neighbouring slots (16 bytes, one sector) and goes on with the rows whose
+// chain is not settled.  The three layouts are one walk: linear tables from
+// the key's hash slot, bucket tables from the first slot of its bucket (keys
+// fill a bucket's slots in order, then the next bucket's), dense tables one
+// slot.  A pair's slot before the key's own can hold the key only in a dense
+// table's header (its base), so the slot at or after it is preferred.
+template <uint32_t R>
+__device__ __forceinline__ uint32_t ws_probe_rows(const ShStep& st, uint64_t hdr, const uint32_t (&v)[R], uint32_t m,
+                                                  uint32_t (&pay)[R], uint64_t pol) {
+    const uint64_t* const ht = st.ht;
+    const uint32_t lay = st.ht_layout, log2cap = st.ht_log2, mask = (1u << log2cap) - 1u;
+    const bool dense = lay == GX_HT_DENSE;
+    uint32_t slot[R];
 #pragma unroll
-    for (uint32_t s = 0; s < NS; ++s) {
-        cd[s] = 0;
-        cv[s] = 0;
-        if (s + 1 < NS && msk[s] == 0) {
-            const uint32_t K = (SIG >> (7 + 4 * s)) & 15u;
-            const ShStep& stp = Q.steps[s];
-            const int32_t v = *(const int32_t*)(sbase + off[s]);
-            cv[s] = v;
-            bool f = !(K & kWkF) || (v >= stp.lo && v <= stp.hi);
-            int32_t pp = v;
-            if ((K & kWkP) && f) {
-                if (stp.ht_layout == GX_HT_DENSE) {  // one read: the table header is cached
-                    const uint64_t hdr = s_hdr[s];
-                    const uint32_t u = (uint32_t)v - (uint32_t)hdr;
-                    f = false;
-                    if (v != kEmptyKey && u < (uint32_t)(hdr >> 32)) {
-                        const unsigned long long e = ws_ld_slot((const unsigned long long*)stp.ht + 1 + u, pol_keep);
-                        f = (int32_t)(uint32_t)e == v;
-                        pp = (int32_t)(uint32_t)(e >> 32);
-                    }
-                } else {
-                    f = ht_probe_any(stp.ht, stp.ht_log2, stp.ht_layout, v, &pp);
-                }
-            }
-            if ((K & kWkD) && f) {
-                cd[s] = (uint32_t)(pp - stp.digit_base);
-                if (cd[s] >= stp.digit_card) {
-                    if (lane == 0) raise_error(kErrInvalid);
-                    f = false;
-                }
-            }
-            if (!f) return 0;  // no row of the tile passes
+    for (uint32_t r = 0; r < R; ++r) {
+        bool out = v[r] == (uint32_t)kEmptyKey;
+        if (dense) {
+            const uint32_t u = v[r] - (uint32_t)hdr;
+            out = out || u >= (uint32_t)(hdr >> 32);
+            slot[r] = 1u + u;
+        } else if (lay == GX_HT_BUCKET) {
+            slot[r] = hash_key32((int32_t)v[r], log2cap - 3) * kBucketSlots;
+        } else {
+            slot[r] = hash_key32((int32_t)v[r], log2cap);
+        }
+        if (out) m &= ~(1u << r);
+    }
+    uint32_t u = m;  // rows whose chain is not settled
+#pragma unroll 1
+    for (uint32_t t = 0; u && t <= mask / 2 + 1; ++t) {
+        ulonglong2 e[R];
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) {
+            asm("" : "=l"(e[r].x), "=l"(e[r].y));  // rows not read keep any value: masked below
+            if ((u >> r) & 1u)
+                asm("ld.global.nc.L2::cache_hint.v2.b64 {%0, %1}, [%2], %3;"
+                    : "=l"(e[r].x), "=l"(e[r].y)
+                    : "l"(ht + (slot[r] & ~1u)), "l"(pol));
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) {
+            const uint32_t bit = 1u << r, kx = (uint32_t)e[r].x, ky = (uint32_t)e[r].y;
+            const bool hit = kx == v[r] || ky == v[r];
+            const bool open = !hit && !dense && ky != (uint32_t)kEmptyKey &&
+                              (kx != (uint32_t)kEmptyKey || (slot[r] & 1u));
+            if ((u & bit) && hit) pay[r] = ky == v[r] ? (uint32_t)(e[r].y >> 32) : (uint32_t)(e[r].x >> 32);
+            if ((u & bit) && !hit && !open) m &= ~bit;
+            if (!open) u &= ~bit;
+            slot[r] = ((slot[r] | 1u) + 1u) & mask;
         }
     }
-    // kWsEvalGroups row groups at a time for scalar plans: their column loads
-    // and first-slot probes are all in flight before any is used (grouped
-    // plans, whose group-table inserts are long inlined loops, run one)
-    constexpr uint32_t H = GR ? 1u : kWsEvalGroups;
+    return m & ~u;
+}
+
+// The last probe step of a signature, plus one (0: none).
+constexpr uint32_t ws_probes_end(uint32_t sig) {
+    uint32_t e = 0;
+    for (uint32_t s = 0; s < (sig & 7); ++s)
+        if ((sig >> (7 + 4 * s)) & kWkP) e = s + 1;
+    return e;
+}
+template <uint32_t SIG>
+constexpr uint32_t kWsProbesEnd = ws_probes_end(SIG);
+
+// Four rows of a column read in place (16-byte aligned), without taking room
+// in L1.  (volatile: the loads of a batch stay together at
+// its start, also when a value is used only after the probes.)
+__device__ __forceinline__ uint4 ws_ld_rows(const uint8_t* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+
+// Elements i .. i + 3 of a bit-packed stream of width w (1..32), plus base:
+// the words that hold them are shifted to the first one's bit once (s below,
+// per lane), after which element k starts at bit k * w in every lane.  Reads
+// at most four words past the last element's.
+__device__ __forceinline__ uint4 ws_unpack4(const uint32_t* words, uint32_t i, uint32_t w, uint32_t base) {
+    const uint32_t bit = i * w, s = bit & 31u;
+    const uint32_t* p = words + (bit >> 5);
+    const uint32_t mask = 0xFFFFFFFFu >> (32 - w);
+    const uint32_t p0 = __ldg(p), p1 = __ldg(p + 1);
+    const uint32_t a0 = __funnelshift_r(p0, p1, s);
+    if (w <= 8)
+        return make_uint4((a0 & mask) + base, ((a0 >> w) & mask) + base, ((a0 >> (2 * w)) & mask) + base,
+                          ((a0 >> (3 * w)) & mask) + base);
+    const uint32_t p2 = __ldg(p + 2), p3 = w > 16 ? __ldg(p + 3) : 0u, p4 = w > 24 ? __ldg(p + 4) : 0u;
+    const uint32_t a1 = __funnelshift_r(p1, p2, s), a2 = __funnelshift_r(p2, p3, s), a3 = __funnelshift_r(p3, p4, s);
+    auto at = [&](uint32_t off) {
+        const uint32_t k = off >> 5;
+        const uint32_t lo = k == 0 ? a0 : k == 1 ? a1 : k == 2 ? a2 : a3;
+        const uint32_t hi = k == 0 ? a1 : k == 1 ? a2 : a3;
+        return (__funnelshift_r(lo, hi, off & 31u) & mask) + base;
+    };
+    return make_uint4((a0 & mask) + base, at(w), at(2 * w), at(3 * w));
+}
+
+// Rows i .. i + 3 of a few-run page, run by run (the decision has checked the
+// header and that the runs add up to the page).
+__device__ __noinline__ uint4 ws_runs4(const uint8_t* pg, uint32_t i) {
+    const casc_hdr h = casc_load_header(pg);
+    const bool delta = (h.flags & CASC_DELTA) != 0;
+    const uint32_t* vw = (const uint32_t*)(pg + h.vals_off);
+    const uint32_t* lw = (const uint32_t*)(pg + h.lens_off);
+    uint32_t start = 0, val = delta ? (uint32_t)h.first : 0u;
+    uint4 v = make_uint4(0, 0, 0, 0);
 #pragma unroll 1
-    for (uint32_t j0 = 0; j0 < kWsGroups; j0 += H) {
-        uint32_t kk[H];
-        uint32_t live = 0;
-#pragma unroll
-        for (uint32_t h = 0; h < H; ++h) {
-            kk[h] = (keep >> (4 * (j0 + h))) & 15u;
-            live |= kk[h];
-        }
-        if (!live) continue;
-        uint4 w[H][NS];
-#pragma unroll
-        for (uint32_t h = 0; h < H; ++h) {
-            const uint32_t ro = (128 * (j0 + h) + 4 * lane) * 4;
-            // (a column constant on the tile reads its broadcast slot: mask 0)
-#pragma unroll
-            for (uint32_t s = 0; s < NS; ++s) w[h][s] = *(const uint4*)(sbase + off[s] + (ro & msk[s]));
-        }
-        int32_t carry[H][4];
-        uint32_t g[H][4];
-#pragma unroll
-        for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                carry[h][i] = 0;
-                g[h][i] = 0;
-            }
+    for (uint32_t k = 0; k < h.n_runs; ++k) {
+        const uint32_t e = (delta && k == 0) ? 0u : unpack_bits(vw, k, h.val_bits) + (uint32_t)h.val_base;
+        val = delta ? val + e : e;
+        if (i >= start) v.x = val;
+        if (i + 1 >= start) v.y = val;
+        if (i + 2 >= start) v.z = val;
+        if (i + 3 >= start) v.w = val;
+        start += unpack_bits(lw, k, h.len_bits) + h.len_base;
+    }
+    return v;
+}
+
+template <uint32_t R>
+__device__ __forceinline__ void ws_put(uint32_t (&w)[R], uint32_t h, const uint4& x) {
+    w[4 * h] = x.x;
+    w[4 * h + 1] = x.y;
+    w[4 * h + 2] = x.z;
+    w[4 * h + 3] = x.w;
+}
+
+// Tile rows row .. row + 3 of a column of two runs.
+__device__ __forceinline__ uint4 ws_runs2(const WsCol& d, uint32_t row) {
+    const uint32_t e = d.aux0, v0 = (uint32_t)d.cval, v1 = d.aux1;
+    return make_uint4(row < e ? v0 : v1, row + 1 < e ? v0 : v1, row + 2 < e ? v0 : v1, row + 3 < e ? v0 : v1);
+}
+
+// Tile rows row .. row + 3 of a column, however it is read.
+__device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
+    const uint32_t mode = d.mode;
+    if (mode == kWmDirect) return ws_ld_rows(d.src + 4 * row);
+    if (mode == kWmPack) return ws_unpack4((const uint32_t*)d.src, d.bytes + row, d.aux0, (uint32_t)d.cval);
+    const uint32_t v0 = (uint32_t)d.cval;
+    if (mode == kWmConst) return make_uint4(v0, v0, v0, v0);
+    if (mode == kWmRuns2) return ws_runs2(d, row);
+    if (mode == kWmRuns) return ws_runs4(d.src, d.bytes + row);
+    return *(const uint4*)(d.src + 4 * row);  // kWmRows
+}
+
+// Tile rows [a, b) evaluated through the plan's steps, H 128-row groups at a
+// time (a is a multiple of kWsPartRows): the lane's rows of group j are
+// 128 j + 4 lane + i (i < 4), row r = 4 h + i of the batch; bit r of m is its
+// mask.  A compile-time signature loads all columns of the batch before any
+// is used and unrolls its steps: up to the last probe step by step, the
+// filters after it and the aggregate row by row, where a row's mask is a
+// predicate.  The run-time form (SIG 0) loads a column at its step.  FLAT:
+// [a, b) is whole batches and every column is direct or a probe's constant or
+// two-run one (a sorted date), so that a batch's loads are unconditional and
+// all in flight together.  Steps over constant columns were decided by
+// ws_const_steps.
+// Returns the scalar part; grouped sums go to the CTA's group table through
+// the warp's queue.
+template <uint32_t SIG, bool FLAT>
+__device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, uint32_t cst, const uint32_t* sdig,
+                                           uint32_t a, uint32_t b, uint32_t* tkey, WsQueue* wq, uint32_t& qn,
+                                           uint64_t pol_keep, const uint64_t* s_hdr,
+                                           uint32_t lane) {
+    constexpr bool GR = SIG == 0 || ((SIG >> 6) & 1) != 0;  // may be grouped: the queue holds one row group
+    constexpr uint32_t H = GR ? 1 : kWsEvalGroups;
+    constexpr uint32_t R = 4 * H;
+    constexpr uint32_t NS = SIG ? (SIG & 7) : 1;
+    constexpr uint32_t PE = SIG ? kWsProbesEnd<SIG> : 0;  // steps [0, PE) run step by step
+    const uint32_t ns = SIG ? NS : Q.n_steps;
+    const uint32_t agg = SIG ? (SIG >> 3) & 7 : Q.agg;
+    const bool grouped = SIG ? ((SIG >> 6) & 1) != 0 : Q.grouped != 0;
+    int64_t acc = 0;
+    const uint8_t* src[NS];  // FLAT: the lane's quad of each step's column
+    uint32_t some = ~0u;     // signatures: 0 when a filter after the probes has an empty range
+    if (SIG) {
 #pragma unroll
         for (uint32_t s = 0; s < NS; ++s) {
-            const uint32_t K = (SIG >> (7 + 4 * s)) & 15u;
+            src[s] = FLAT ? cols[Q.steps[s].col].src + (a + 4 * lane) * 4 : nullptr;
+            if (s >= PE && ((SIG >> (7 + 4 * s)) & kWkF) && Q.steps[s].lo > Q.steps[s].hi) some = 0;
+        }
+    }
+#pragma unroll 1
+    for (uint32_t j0 = a; j0 < b; j0 += H * kWsBatch) {
+        const uint32_t row = j0 + 4 * lane;
+        uint32_t m = (1u << R) - 1u;
+        if (!FLAT && j0 + H * kWsBatch > b) {
+            m = 0;
+#pragma unroll
+            for (uint32_t r = 0; r < R; ++r)
+                if (row + kWsBatch * (r / 4) + r % 4 < b) m |= 1u << r;
+        }
+        uint32_t w[NS][R];
+        uint32_t g[R], carry[R];
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) g[r] = carry[r] = 0;
+        if (SIG) {
+            // (values of rows that are not wanted are not used: any will do.  A quad with one
+            // wanted row ends at most 12 bytes after its block, inside the payload)
+#pragma unroll
+            for (uint32_t s = 0; s < NS; ++s) {
+                const bool skip = ((SIG >> (7 + 4 * s)) & kWkP) && ((cst >> s) & 1u);
+#pragma unroll
+                for (uint32_t h = 0; h < H; ++h) {
+                    uint4 x;
+                    asm("" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w));
+                    if (FLAT) {
+                        const WsCol& d = cols[Q.steps[s].col];
+                        if (((SIG >> (7 + 4 * s)) & kWkP) && !skip && d.mode == kWmRuns2)
+                            x = ws_runs2(d, row + kWsBatch * h);
+                        else if (!skip)
+                            x = ws_ld_rows(src[s] + kWsBatch * 4 * h);
+                    } else if (cols[Q.steps[s].col].mode == kWmDirect && row + kWsBatch * h < b) {
+                        x = ws_ld_rows(cols[Q.steps[s].col].src + (row + kWsBatch * h) * 4);
+                    }
+                    ws_put(w[s], h, x);
+                }
+                if (FLAT) src[s] += H * kWsBatch * 4;
+            }
+            if (!FLAT) {
+#pragma unroll
+                for (uint32_t s = 0; s < NS; ++s) {
+                    const WsCol& d = cols[Q.steps[s].col];
+                    if (d.mode == kWmDirect) continue;
+#pragma unroll
+                    for (uint32_t h = 0; h < H; ++h)
+                        if (row + kWsBatch * h < b) ws_put(w[s], h, ws_quad(d, row + kWsBatch * h));
+                }
+            }
+        }
+        // one step over the batch: v = the lane's rows of its column
+        auto step = [&](uint32_t s, uint32_t K, const uint32_t (&v)[R]) {
             const ShStep& stp = Q.steps[s];
-            if (s + 1 < NS && msk[s] == 0) {  // decided for the tile
-                if (K & kWkD) {
-                    const uint32_t dcard = stp.digit_card;
-#pragma unroll
-                    for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) g[h][i] = g[h][i] * dcard + cd[s];
-                }
-                if (K & kWkC) {
-#pragma unroll
-                    for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) carry[h][i] = cv[s];
-                }
-                continue;
-            }
-            int32_t v[H][4];
-#pragma unroll
-            for (uint32_t h = 0; h < H; ++h) {
-                v[h][0] = (int32_t)w[h][s].x;
-                v[h][1] = (int32_t)w[h][s].y;
-                v[h][2] = (int32_t)w[h][s].z;
-                v[h][3] = (int32_t)w[h][s].w;
-            }
-            if (K & kWkF) {
+            const bool decided = ((cst >> s) & 1u) != 0;
+            if ((K & kWkF) && !decided) {
                 // lo <= v <= hi as one unsigned comparison of v - lo with hi - lo
                 // (an empty range, hi < lo, keeps nothing)
                 const uint32_t lo = (uint32_t)stp.lo, span = (uint32_t)stp.hi - lo;
-                const uint32_t none = stp.hi < stp.lo ? 0u : 15u;
+                if (stp.lo > stp.hi) m = 0;
 #pragma unroll
-                for (uint32_t h = 0; h < H; ++h) {
-                    uint32_t pass = 0;
-#pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) pass |= ((uint32_t)v[h][i] - lo <= span) ? 1u << i : 0u;
-                    kk[h] &= pass & none;
-                }
+                for (uint32_t r = 0; r < R; ++r)
+                    if (v[r] - lo > span) m &= ~(1u << r);
             }
-            int32_t pp[H][4];
+            uint32_t pp[R];
 #pragma unroll
-            for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) pp[h][i] = v[h][i];
-            if (K & kWkP) {
-                const uint64_t* const ht = stp.ht;
-                const uint32_t htlog = stp.ht_log2, htlay = stp.ht_layout;
-                const bool dense = htlay == GX_HT_DENSE, bucket = htlay == GX_HT_BUCKET;
-                uint32_t hbase = 0, hspan = 0;
-                if (dense) {
-                    const uint64_t hdr = s_hdr[s];
-                    hbase = (uint32_t)hdr;
-                    hspan = (uint32_t)(hdr >> 32);
-                }
-                // the first slot of every kept row's key, all read before any is used
-                uint64_t ee[H][4];
-#pragma unroll
-                for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) {
-                        const uint32_t u = (uint32_t)v[h][i] - hbase;
-                        const bool r =
-                            ((kk[h] >> i) & 1u) && !bucket && v[h][i] != kEmptyKey && (!dense || u < hspan);
-                        const unsigned long long* sl =
-                            (const unsigned long long*)ht + (dense ? 1 + u : hash_key32(v[h][i], htlog));
-                        ee[h][i] = r ? ws_ld_slot(sl, pol_keep) : (unsigned long long)kEmptySlot;
-                    }
-#pragma unroll
-                for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) {
-                        if (!((kk[h] >> i) & 1u)) continue;
-                        const int32_t ek = (int32_t)(uint32_t)ee[h][i];
-                        bool f;
-                        int32_t p = v[h][i];
-                        if (ek == v[h][i] && v[h][i] != kEmptyKey) {
-                            f = true;
-                            p = (int32_t)(uint32_t)(ee[h][i] >> 32);
-                        } else if (!bucket && (dense || ek == kEmptyKey)) {
-                            f = false;  // an empty first slot, or a dense table's slot of another key
-                        } else {
-                            f = sh_probe(ht, htlog, htlay, v[h][i], &p);  // a linear chain, or a bucket table
-                        }
-                        pp[h][i] = p;
-                        if (!f) kk[h] &= ~(1u << i);
-                    }
-            }
+            for (uint32_t r = 0; r < R; ++r) pp[r] = v[r];
+            if ((K & kWkP) && !decided) m = ws_probe_rows<R>(stp, s_hdr[s], v, m, pp, pol_keep);
             if (K & kWkD) {
-                const uint32_t dcard = stp.digit_card;
-                const int32_t dbase = stp.digit_base;
-#pragma unroll
-                for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) {
-                        if (!((kk[h] >> i) & 1u)) continue;
-                        const uint32_t dgt = (uint32_t)(pp[h][i] - dbase);
-                        if (dgt >= dcard) {
-                            raise_error(kErrInvalid);
-                            kk[h] &= ~(1u << i);
-                        } else {
-                            g[h][i] = g[h][i] * dcard + dgt;
-                        }
+                const uint32_t dcard = stp.digit_card, dbase = (uint32_t)stp.digit_base, cdig = sdig[s];
+                if (decided) {  // (run-time form: kWsNone, a digit out of range)
+                    if (SIG == 0 && cdig >= dcard && m) {
+                        raise_error(kErrInvalid);
+                        m = 0;
                     }
+#pragma unroll
+                    for (uint32_t r = 0; r < R; ++r) g[r] = g[r] * dcard + cdig;
+                } else {
+                    uint32_t bad = 0;
+#pragma unroll
+                    for (uint32_t r = 0; r < R; ++r) {
+                        const uint32_t dgt = pp[r] - dbase;
+                        if (dgt >= dcard) bad |= 1u << r;
+                        g[r] = g[r] * dcard + dgt;
+                    }
+                    if (bad & m) {
+                        raise_error(kErrInvalid);
+                        m &= ~bad;
+                    }
+                }
             }
             if (K & kWkC) {
 #pragma unroll
-                for (uint32_t h = 0; h < H; ++h)
-#pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) carry[h][i] = v[h][i];
+                for (uint32_t r = 0; r < R; ++r) carry[r] = v[r];
             }
-            live = 0;
+        };
+        uint32_t val[R];  // the last column
+        if constexpr (SIG != 0) {
 #pragma unroll
-            for (uint32_t h = 0; h < H; ++h) live |= kk[h];
-            if (!live) break;
-            if (s + 1 == NS) {
+            for (uint32_t s = 0; s < NS; ++s) {
+                const uint32_t K = (SIG >> (7 + 4 * s)) & 15u;
+                if (s < PE || (K & kWkD)) step(s, K, w[s]);
+                else if (K & kWkC) {
+#pragma unroll
+                    for (uint32_t r = 0; r < R; ++r) carry[r] = w[s][r];
+                }
+            }
+            m &= some;
+#pragma unroll
+            for (uint32_t r = 0; r < R; ++r) val[r] = w[NS - 1][r];
+        } else {
+#pragma unroll
+            for (uint32_t r = 0; r < R; ++r) val[r] = 0;
+#pragma unroll 1
+            for (uint32_t s = 0; s < ns; ++s) {
+                if (!__any_sync(0xFFFFFFFFu, m)) break;
+                const ShStep& stp = Q.steps[s];
+                const WsCol& d = cols[stp.col];
 #pragma unroll
                 for (uint32_t h = 0; h < H; ++h) {
-                    if (GR) {
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) {
-                            if (!((kk[h] >> i) & 1u)) continue;
-                            const int64_t val = AGG == GX_AGG_SUM_PRODUCT ? (int64_t)v[h][i] * carry[h][i]
-                                                : AGG == GX_AGG_SUM_DIFF  ? (int64_t)v[h][i] - carry[h][i]
-                                                : AGG == GX_AGG_COUNT      ? 1
-                                                                           : (int64_t)v[h][i];
-                            ws_group_add(g[h][i], val, tkey, tsum, Q.g_keys, Q.g_sums, Q.g_log2);
-                        }
-                    } else {
-                        // kept rows as multiply-adds by 0 or 1 (one wide multiply-add per row)
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) {
-                            const int32_t on = (int32_t)((kk[h] >> i) & 1u);
-                            if (AGG == GX_AGG_SUM_PRODUCT) {
-                                acc += (int64_t)v[h][i] * (int64_t)(on ? carry[h][i] : 0);
-                            } else if (AGG == GX_AGG_SUM_DIFF) {
-                                acc += (int64_t)v[h][i] * on;
-                                acc -= (int64_t)carry[h][i] * on;
-                            } else if (AGG == GX_AGG_COUNT) {
-                                acc += on;
-                            } else {
-                                acc += (int64_t)v[h][i] * on;
-                            }
-                        }
-                    }
+                    uint4 x = make_uint4(0, 0, 0, 0);
+                    if (row + kWsBatch * h < b) x = ws_quad(d, row + kWsBatch * h);
+                    ws_put(val, h, x);
                 }
+                const uint32_t f = stp.flags;
+                step(s, ((f & GX_STEP_FILTER) ? kWkF : 0u) | ((f & GX_STEP_PROBE) ? kWkP : 0u) |
+                            ((f & GX_STEP_CARRY) ? kWkC : 0u) | (stp.digit_card ? kWkD : 0u), val);
+            }
+        }
+        // the filters after the probes and the aggregate, row by row
+        auto kept = [&](uint32_t r) {
+            bool k = ((m >> r) & 1u) != 0;
+            if (SIG) {
+#pragma unroll
+                for (uint32_t s = PE; s < NS; ++s)
+                    if ((SIG >> (7 + 4 * s)) & kWkF) {
+                        const uint32_t lo = (uint32_t)Q.steps[s].lo, span = (uint32_t)Q.steps[s].hi - lo;
+                        k = k && w[s][r] - lo <= span;
+                    }
+            }
+            return k;
+        };
+        auto value = [&](uint32_t r) -> int64_t {
+            const int32_t x = (int32_t)val[r], c = (int32_t)carry[r];
+            return agg == GX_AGG_SUM_PRODUCT ? (int64_t)x * c
+                   : agg == GX_AGG_SUM_DIFF  ? (int64_t)x - c
+                   : agg == GX_AGG_COUNT     ? 1
+                                             : (int64_t)x;
+        };
+        if (!grouped) {
+#pragma unroll
+            for (uint32_t r = 0; r < R; ++r) {
+                if constexpr (SIG == kSigQ1) {
+                    // both filters and the multiply-add as one predicate chain
+                    asm("{\n .reg .pred p;\n .reg .u32 d, e;\n sub.u32 d, %1, %2;\n sub.u32 e, %4, %5;\n"
+                        " setp.ne.u32 p, %7, 0;\n setp.le.and.u32 p, d, %3, p;\n setp.le.and.u32 p, e, %6, p;\n"
+                        " @p mad.wide.s32 %0, %8, %9, %0;\n}"
+                        : "+l"(acc)
+                        : "r"(w[1][r]), "r"(Q.steps[1].lo), "r"((uint32_t)Q.steps[1].hi - (uint32_t)Q.steps[1].lo),
+                          "r"(w[2][r]), "r"(Q.steps[2].lo), "r"((uint32_t)Q.steps[2].hi - (uint32_t)Q.steps[2].lo),
+                          "r"(m & (1u << r)), "r"(w[3][r]), "r"(w[1][r]));
+                } else if (kept(r)) {
+                    acc += value(r);
+                }
+            }
+        } else {
+            const uint32_t below = (1u << lane) - 1u;
+#pragma unroll
+            for (uint32_t r = 0; r < R; ++r) {
+                const bool on = kept(r);
+                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+                if (__popc(bal) >= 24) {  // most lanes have a row: no detour through the queue
+                    ws_group_add_lanes(on, g[r], value(r), tkey, Q.g_keys, Q.g_sums, Q.g_log2);
+                    continue;
+                }
+                if (on) {
+                    const uint32_t at = qn + __popc(bal & below);
+                    wq->key[at] = g[r];
+                    wq->val[at] = value(r);
+                }
+                qn += __popc(bal);
+            }
+            while (qn >= 32) {
+                qn -= 32;
+                ws_queue_flush(wq, qn, 32, tkey, Q.g_keys, Q.g_sums, Q.g_log2, lane);
             }
         }
     }
     return acc;
 }
 
+// The general evaluator out of line: ragged tiles, columns that are not
+// direct, run-time plans.
 template <uint32_t SIG>
-__global__ void __launch_bounds__(kWsNT, (SIG == 0 || ((SIG >> 6) & 1)) ? 4 : 3) warp_scan_kernel(const __grid_constant__ WsParams P) {
+__device__ __noinline__ int64_t ws_eval_any(const ShQuery& Q, const WsCol* cols, uint32_t cst, const uint32_t* sdig,
+                                            uint32_t a, uint32_t b, uint32_t* tkey, WsQueue* wq, uint32_t* qn,
+                                            uint64_t pol_keep, const uint64_t* s_hdr,
+                                            uint32_t lane) {
+    uint32_t n = *qn;
+    const int64_t acc = ws_eval<SIG, false>(Q, cols, cst, sdig, a, b, tkey, wq, n, pol_keep, s_hdr, lane);
+    *qn = n;
+    return acc;
+}
+
+// CTAs per SM each form is built for.  Scalar signatures (two row groups and
+// their columns in registers) keep 96 registers: five CTAs, 20 warps, scan Q1
+// over 60M rows in 132 us where four take 165 us (too few loads in flight) and
+// six 150 us (spills).  Grouped ones (one row group, probes) take six: the
+// 200M-row star join 2.17 ms, 2.26 with five, 2.35 with seven.  Run-time plans
+// wait on group-table adds and take eight (778 us against 909 us with five,
+// 30M rows into 1.4M groups).
+constexpr int ws_ctas(uint32_t sig) { return sig == 0 ? 8 : ((sig >> 6) & 1) ? 6 : 5; }
+
+template <uint32_t SIG>
+__global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __grid_constant__ WsParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ gx_dcol s_cols[kWsMaxCols];
-    __shared__ uint32_t s_nsurv;
+    __shared__ WsWork s_work;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ncols = P.n_cols;
     const ShQuery& Q = P.q;
     uint32_t* const s_kbits = (uint32_t*)smem;               // chunk keep bits of [chunk_lo, chunk_hi)
     uint32_t* const s_kpre = s_kbits + P.chunk_words;        // surviving chunks before each word
     uint32_t* const wmem = s_kpre + P.chunk_words + (size_t)warp * P.warp_words;
-    uint4* const cslot = (uint4*)wmem;                       // constant columns (4 copies of the value)
-    uint64_t* const bar = (uint64_t*)(wmem + 4 * kWsMaxCols);  // the warp's stage mbarrier
-    uint64_t* const whdr = (uint64_t*)(wmem + 4 * kWsMaxCols + 4);  // dense join tables' headers, per step
-    uint32_t* const areas = wmem + kWsHead;                  // n_areas x kWsTile words
-    // grouped plans: the run-time evaluator's group key of each row of the tile
-    // (compile-time evaluators keep keys in registers), then the group table
-    uint32_t* const gkb = areas + (size_t)P.n_areas * kWsTile;
-    // grouped: the CTA's group table (keys, then sums) after the warps' regions
+    WsCol* const wcols = (WsCol*)wmem;                       // column records of the round's tiles
+    WsTile* const wtiles = (WsTile*)(wmem + 32 * 8);         // their tile records
+    uint64_t* const whdr = (uint64_t*)(wmem + 40 * 8);  // dense join tables' headers, per step
+    uint32_t* const wdig = wmem + 40 * 8 + 2 * GX_MAX_STEPS;  // constant steps' group-key digits
+    unsigned long long* const wrows = (unsigned long long*)(wdig + 32);  // rows scanned
+    WsQueue* const wq = (WsQueue*)(wmem + kWsHead);          // grouped: rows on their way to the group table
+    uint32_t* const areas = wmem + kWsHead + (P.grouped_tab ? kWsQueueWords : 0u);  // n_areas x kWsTile words
+    // grouped: the CTA's group table (keys, low halves, high halves of the sums) after the warps' regions
     uint32_t* const tkey = s_kpre + P.chunk_words + (size_t)kWsWarps * P.warp_words;
-    unsigned long long* const tsum = (unsigned long long*)(tkey + kWsGroupSlots);
-    const uint64_t pol_keep = ws_policy_keep(), pol_stream = ws_policy_stream();
+    const uint64_t pol_keep = ws_policy_keep();
 
     // The launch may overlap the kernel before it on the stream (programmatic
     // dependent launch): until a thread has passed griddep_wait it reads only
@@ -946,210 +1098,138 @@ __global__ void __launch_bounds__(kWsNT, (SIG == 0 || ((SIG >> 6) & 1)) ? 4 : 3)
         const uint32_t word = __ballot_sync(0xFFFFFFFFu, ck);
         if (lane == 0) s_kbits[wb / 32] = word;
     }
-    if (lane == 0) mbar_init(bar, 1);
     if (P.grouped_tab) {
         for (uint32_t i = tid; i < kWsGroupSlots; i += kWsNT) {
             tkey[i] = kEmptyGKey;
-            tsum[i] = 0;
+            tkey[kWsGroupSlots + i] = 0;
+            tkey[2 * kWsGroupSlots + i] = 0;
         }
     }
     __syncthreads();
     if (warp == 0) {  // exclusive prefix of the popcounts: per lane a run of words, then a warp scan
         const uint32_t per = (P.chunk_words + 31) / 32, w0 = min(P.chunk_words, lane * per),
                        w1 = min(P.chunk_words, w0 + per);
-        uint32_t cnt = 0;
-        for (uint32_t i = w0; i < w1; ++i) cnt += __popc(s_kbits[i]);
+        uint32_t cnt = 0, first = kWsNone, last = 0;  // surviving chunks of the lane's words: count, first, last
+        for (uint32_t i = w0; i < w1; ++i) {
+            const uint32_t m = s_kbits[i];
+            cnt += __popc(m);
+            if (m) {
+                first = min(first, i * 32 + (__ffs(m) - 1));
+                last = i * 32 + (31 - __clz(m));
+            }
+        }
         uint32_t run = ws_scan(cnt, lane) - cnt;
         for (uint32_t i = w0; i < w1; ++i) {
             s_kpre[i] = run;
             run += __popc(s_kbits[i]);
         }
-        if (lane == 31) s_nsurv = run;
+        first = __reduce_min_sync(0xFFFFFFFFu, first);
+        last = __reduce_max_sync(0xFFFFFFFFu, last);
+        if (lane == 31) {
+            WsWork R;
+            R.first = run && last - first + 1 == run ? P.chunk_lo + first : kWsNone;
+            R.t_end = run * P.blocks_per_chunk * P.tiles_per_block;  // the launch keeps tile indices below 2^31
+            R.W = gridDim.x * kWsWarps;
+            R.full = R.t_end / R.W;
+            const uint32_t left = R.t_end - R.full * R.W;
+            R.rounds = R.full + (left ? 1u : 0u);
+            R.parts_log2 = 0;
+            if (P.parts)  // as many parts as there are warps for
+                while ((1u << R.parts_log2) < kWsMaxParts && (left << (R.parts_log2 + 1)) <= R.W) ++R.parts_log2;
+            s_work = R;
+        }
     }
     __syncthreads();  // the last block-wide barrier: warps are independent from here on
 
-    const uint32_t PC = P.blocks_per_chunk * P.tiles_per_block;
-    const uint32_t t_end = s_nsurv * PC;
-    const uint32_t ns = Q.n_steps, agg = Q.agg;
-    const bool grouped = Q.grouped != 0;
-    const uint32_t W = gridDim.x * kWsWarps;
+    const uint32_t w = blockIdx.x * kWsWarps + warp, rounds = s_work.rounds;
     int64_t local = 0;
-    unsigned long long local_rows = 0;
-    uint32_t ph = 0;
-    bool stop = false;
-    for (uint32_t t0 = blockIdx.x * kWsWarps + warp; t0 < t_end && !stop; t0 += 4 * W) {
-        WsTile T;
-        WsCol C;
-        const uint32_t vm = ws_decide(P, s_cols, s_kbits, s_kpre, t0, W, t_end, lane, T, C);
-        ws_prefetch_meta(P, s_cols, s_kbits, s_kpre, t0 + 4 * W, W, t_end, lane);
-        // the staged ranges of every tile of the four go to L2 now
-        if (((vm >> (lane >> 3)) & 1u) && (lane & 7) < ncols && C.mode == kWmStage) ws_bulk_prefetch_l2(C.src, C.bytes, pol_stream);
-        for (uint32_t q = 0; q < 4 && !stop; ++q) {
+    uint32_t qn = 0;  // rows in the warp's queue
+    if (lane == 0) *wrows = 0;
+    const uint32_t cl = P.col_log2, nq = 32u >> cl;
+    for (uint32_t r0 = 0; r0 < rounds; r0 += nq) {
+        const uint32_t vm = ws_decide(P, s_cols, s_kbits, s_kpre, s_work, w, r0, lane, wtiles, wcols);
+        if (!vm) continue;
+        if (!tables) {
+            await_tables();
+            tables = true;
+        }
+        ws_const_steps<SIG>(P, vm, wtiles, wcols, whdr, wdig, pol_keep, lane);
+        for (uint32_t q = 0; q < nq; ++q) {
             if (!((vm >> q) & 1u)) continue;
-            const uint32_t L0 = 8 * q, Lc = 8 * q + (lane & 7);
-            const uint32_t slot = __shfl_sync(0xFFFFFFFFu, T.slot, L0), r0 = __shfl_sync(0xFFFFFFFFu, T.r0, L0);
-            const uint32_t n = __shfl_sync(0xFFFFFFFFu, T.n, L0), rows = __shfl_sync(0xFFFFFFFFu, T.rows, L0);
-            const uint32_t a = __shfl_sync(0xFFFFFFFFu, T.a, L0), b = __shfl_sync(0xFFFFFFFFu, T.b, L0);
-            // lane c (< ncols): column c of this tile
-            const uint32_t mode = __shfl_sync(0xFFFFFFFFu, C.mode, Lc);
-            const uint8_t* src = (const uint8_t*)ws_shfl64((uint64_t)C.src, Lc);
-            const uint32_t aux0 = __shfl_sync(0xFFFFFFFFu, C.aux0, Lc), aux1 = __shfl_sync(0xFFFFFFFFu, C.aux1, Lc);
-            const uint32_t cbytes = __shfl_sync(0xFFFFFFFFu, C.bytes, Lc);
-            const int32_t cval = (int32_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)C.cval, Lc);
-            const bool mine = lane < ncols;
-            // ---- stage copies (one bulk copy per in-place column)
-            const uint32_t my = (mine && mode == kWmStage) ? cbytes : 0u;
-            const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, my);
-            if (total) {
-                if (lane == 0) mbar_expect_tx_arrive(bar, total);
-                __syncwarp();
-                if (my) ws_bulk_copy(areas + (size_t)P.stage_of[lane] * kWsTile, src, my, bar, pol_stream);
-            }
+            const WsTile& T = wtiles[q];
+            WsCol* const cols = wcols + (q << cl);
             // ---- decodes, one column at a time by the whole warp
-            int terr = __any_sync(0xFFFFFFFFu, mine && mode == kWmBad) ? kErrCorrupt : 0;
-            uint32_t roff = 0, rmask = 0xFFFFFFFFu;  // lane c: shared-memory byte offset of column c's rows
-            if (mine) {
-                if (mode == kWmStage) {
-                    roff = (uint32_t)((uint8_t*)(areas + (size_t)P.stage_of[lane] * kWsTile) - smem);
-                } else if (mode == kWmConst) {
-                    cslot[lane] = make_uint4((uint32_t)cval, (uint32_t)cval, (uint32_t)cval, (uint32_t)cval);
-                    roff = (uint32_t)((uint8_t*)&cslot[lane] - smem);
-                    rmask = 0;
-                }
-            }
-            for (uint32_t c = 0; c < ncols && !terr; ++c) {
-                const uint32_t m = __shfl_sync(0xFFFFFFFFu, mode, c);
-                if (m != kWmLz4 && m != kWmCasc && m != kWmRuns2) continue;
-                uint32_t* buf = areas + (size_t)P.buf_of[c] * kWsTile;
-                if (m == kWmRuns2) {  // two runs: the rows written out directly
-                    const uint32_t v0 = (uint32_t)__shfl_sync(0xFFFFFFFFu, (uint32_t)cval, c);
-                    const uint32_t split = __shfl_sync(0xFFFFFFFFu, aux0, c), v1 = __shfl_sync(0xFFFFFFFFu, aux1, c);
-#pragma unroll 1
-                    for (uint32_t j = 0; j < kWsTile / 128; ++j) {
-                        const uint32_t r = 128 * j + 4 * lane;
-                        *(uint4*)(buf + r) = make_uint4(r < split ? v0 : v1, r + 1 < split ? v0 : v1,
-                                                        r + 2 < split ? v0 : v1, r + 3 < split ? v0 : v1);
-                    }
-                    __syncwarp();
-                    if (lane == c) roff = (uint32_t)((uint8_t*)buf - smem);
-                    continue;
-                }
-                const uint8_t* cs = (const uint8_t*)ws_shfl64((uint64_t)src, c);
-                const uint32_t x0 = __shfl_sync(0xFFFFFFFFu, aux0, c), x1 = __shfl_sync(0xFFFFFFFFu, aux1, c);
-                int r;
-                int32_t cv = 0;
-                if (m == kWmCasc) {
-                    r = ws_casc_rows(cs, x0, x1, r0 & (kCascPageRows - 1u), n, (int32_t*)buf, &cv, lane);
-                } else {
-                    const uint32_t bb = __shfl_sync(0xFFFFFFFFu, cbytes, c);
-                    const gx_dcol& col = s_cols[c];
-                    r = ws_lz4_rows(cs, bb, col.seg + (size_t)2 * col.S * slot, col.seg_shift, rows, r0, n, x0, x1,
-                                    buf, lane);
-                }
-                if (r == 1) {  // one value for the whole tile
-                    if (lane == c) {
-                        cslot[c] = make_uint4((uint32_t)cv, (uint32_t)cv, (uint32_t)cv, (uint32_t)cv);
-                        roff = (uint32_t)((uint8_t*)&cslot[c] - smem);
-                        rmask = 0;
-                    }
-                } else if (r) {
-                    terr = r;
-                } else if (lane == c) {
-                    roff = (uint32_t)((uint8_t*)buf - smem);
-                }
-            }
-            // ---- the staged bytes
-            if (total) {
-                const bool ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, ph));
-                ph ^= 1u;
-                if (!ok) {
-                    // the copies did not land: stop this warp (after one more bounded
-                    // wait, so that no copy is left in flight into its shared memory)
-                    if (lane == 0) raise_error(kErrTimeout);
-                    mbar_wait_bounded(bar, ph ^ 1u);
-                    stop = true;
+            int terr = 0;
+            for (uint32_t c = 0; c < ncols; ++c) {
+                const uint32_t m = cols[c].mode;
+                if (m == kWmBad) {
+                    terr = kErrCorrupt;
                     break;
                 }
+                if (m != kWmLz4 && m != kWmCasc) continue;
+                uint32_t* buf = areas + (size_t)P.buf_of[c] * kWsTile;
+                int32_t cv = 0;
+                int r = 0;
+                if (m == kWmCasc) {
+                    r = ws_casc_rows(cols[c].src, cols[c].aux0, cols[c].aux1, T.r0 & (kCascPageRows - 1u), T.n,
+                                     (int32_t*)buf, &cv, lane);
+                    if (r == 1) {  // one run covers the tile (a page of many runs): its value written out
+                        for (uint32_t i = lane; i < T.n; i += 32) buf[i] = (uint32_t)cv;
+                        r = 0;
+                    }
+                } else {
+                    const gx_dcol& col = s_cols[c];
+                    r = ws_lz4_rows(cols[c].src, cols[c].bytes, col.seg + (size_t)2 * col.S * T.slot, col.seg_shift,
+                                    T.rows, T.r0, T.n, cols[c].aux0, cols[c].aux1, buf, lane);
+                }
+                __syncwarp();
+                if (r) {
+                    terr = r;
+                    break;
+                }
+                if (lane == 0) {
+                    cols[c].mode = kWmRows;
+                    cols[c].src = (const uint8_t*)buf;
+                }
+                __syncwarp();
             }
-            __syncwarp();
             if (terr) {
                 if (lane == 0) raise_error(terr);
-            } else {
-                local_rows += b - a;  // lane-uniform; lane 0's count is the warp's
-                // ---- evaluation, step-major over the tile: the lane's rows are
-                // 128 j + 4 lane + i (j < kWsGroups, i < 4), keep bit 4 j + i
-                uint32_t keep = kWsGroups == 8 ? 0xFFFFFFFFu : (1u << (4 * kWsGroups)) - 1u;
-                if (a != 0 || b != kWsTile) {
-                    keep = 0;
-#pragma unroll 1
-                    for (uint32_t j = 0; j < kWsGroups; ++j) {
-                        const int32_t base = (int32_t)(128 * j + 4 * lane);
-                        const int32_t l = min(4, max(0, (int32_t)a - base)), h = min(4, max(0, (int32_t)b - base));
-                        keep |= (h > l ? ((1u << h) - 1u) & ~((1u << l) - 1u) : 0u) << (4 * j);
-                    }
-                }
-                if (SIG == 0 && grouped) {
-#pragma unroll 1
-                    for (uint32_t j = 0; j < kWsGroups; ++j) *(uint4*)(gkb + 128 * j + 4 * lane) = make_uint4(0, 0, 0, 0);
-                }
-                if (!tables) {
-                    await_tables();
-                    tables = true;
-                }
-                if constexpr (SIG != 0) {
-                    constexpr uint32_t NS = SIG & 7;
-                    uint32_t off[NS], msk[NS];
-#pragma unroll
-                    for (uint32_t s = 0; s < NS; ++s) {
-                        const uint32_t c = Q.steps[s].col;
-                        off[s] = __shfl_sync(0xFFFFFFFFu, roff, c);
-                        msk[s] = __shfl_sync(0xFFFFFFFFu, rmask, c);
-                    }
-                    local += ws_eval_sig<SIG>(Q, smem, off, msk, keep, tkey, tsum, pol_keep, whdr, lane);
-                }
-                uint32_t coff = 0, cmask = 0;  // the carried column (none: carried values are 0)
-                bool carried = false;
-                for (uint32_t s = 0; SIG == 0 && s < ns; ++s) {
-                    if (!__any_sync(0xFFFFFFFFu, keep)) break;
-                    const ShStep& stp = Q.steps[s];
-                    const uint32_t flags = stp.flags;
-                    const uint32_t c = stp.col;
-                    const uint32_t off = __shfl_sync(0xFFFFFFFFu, roff, c), msk = __shfl_sync(0xFFFFFFFFu, rmask, c);
-                    if (flags & GX_STEP_CARRY) {
-                        coff = off;
-                        cmask = msk;
-                        carried = true;
-                    }
-                    if (msk == 0) {
-                        if (ws_step_const(stp, *(const int32_t*)(smem + off), keep, gkb, grouped, lane)) keep = 0;
-                    } else if ((flags & (GX_STEP_FILTER | GX_STEP_PROBE)) || stp.digit_card) {
-                        keep = ws_step_rows(stp, smem + off, keep, gkb, grouped, pol_keep, lane);
-                    }
-                    if (s + 1 == ns && keep)
-                        local += ws_aggregate(agg, grouped, carried, smem + off, msk, smem + coff, cmask, keep, gkb,
-                                              tkey, tsum, Q.g_keys, Q.g_sums, Q.g_log2, lane);
-                }
+                continue;
             }
-            // every lane is done with the tile's areas before the next copies overwrite them
-            __syncwarp();
-            if (lane == 0) fence_proxy_async_smem();
+            if (lane == 0) *wrows += T.b - T.a;
+            // ---- evaluation
+            const uint32_t st = T.steps;
+            if (!(st & kWsDead)) {
+                // whole row batches of direct columns: the flat form
+                const uint32_t* const dig = wdig + (q << cl);
+                if (SIG != 0 && !(st & kWsMixed) && ((T.b - T.a) & (kWsPartRows - 1u)) == 0)
+                    local += ws_eval<SIG, SIG != 0>(Q, cols, st, dig, T.a, T.b, tkey, wq, qn, pol_keep, whdr,
+                                                     lane);
+                else
+                    local += ws_eval_any<SIG>(Q, cols, st, dig, T.a, T.b, tkey, wq, &qn, pol_keep, whdr, lane);
+            }
+            __syncwarp();  // every lane is done with the tile's buffers and records before they are overwritten
         }
+        __syncwarp();
     }
     // ---- results: the CTA's group table once every warp is done, else the warp's sum
+    if (qn) ws_queue_flush(wq, 0, qn, tkey, Q.g_keys, Q.g_sums, Q.g_log2, lane);
     __syncwarp();
     if (!waited) griddep_wait();
     if (blockIdx.x == 0 && Q.keep_out)
         for (uint32_t i = tid; i < n_range; i += kWsNT) Q.keep_out[P.chunk_lo + i] = (s_kbits[i / 32] >> (i % 32)) & 1u;
-    if (grouped && P.grouped_tab) {
+    if (Q.grouped && P.grouped_tab) {
         __syncthreads();
         for (uint32_t i = tid; i < kWsGroupSlots; i += kWsNT) {
             const uint32_t key = tkey[i];
-            if (key != kEmptyGKey && !group_add_global(Q.g_keys, Q.g_sums, Q.g_log2, (int64_t)key, (int64_t)tsum[i]))
+            const uint64_t sum = ((uint64_t)tkey[2 * kWsGroupSlots + i] << 32) | tkey[kWsGroupSlots + i];
+            if (key != kEmptyGKey && !group_add_global(Q.g_keys, Q.g_sums, Q.g_log2, (int64_t)key, (int64_t)sum))
                 raise_error(kErrCapacity);
         }
-    } else if (!grouped) {
+    } else if (!Q.grouped) {
         const uint64_t u = warp_sum_u64((uint64_t)local);
         if (lane == 0 && u && Q.result) atomicAdd((unsigned long long*)Q.result, (unsigned long long)u);
     }
-    if (lane == 0 && P.rows_scanned && local_rows) atomicAdd(P.rows_scanned, local_rows);
+    if (lane == 0 && P.rows_scanned && *wrows) atomicAdd(P.rows_scanned, *wrows);
 }

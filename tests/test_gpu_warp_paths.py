@@ -1,0 +1,94 @@
+"""The warp-tile scan's read paths at their edges, against numpy on the same
+columns: bit-packed pages of every word-straddling width, pages of a few runs
+(more than two on a tile), ragged tiles, chains of nearly full join tables, and
+group keys that overflow the CTA's table."""
+import numpy as np
+import pytest
+
+from golap_public_b200 import _lib as L
+from golap_public_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _warp_form():
+    api.set_scan_form("warp")
+    yield
+    api.set_scan_form("auto")
+
+
+def _col(v, codec, **kw):
+    return api.Column(v.astype(np.int32), codec, rows_per_chunk=40_000, **kw).to_device()
+
+
+def _sum(torch, filt, lo, hi, value, carry=None):
+    res = torch.zeros(1, dtype=torch.int64, device="cuda")
+    p = api.ScanPlan(agg=L.GX_AGG_SUM_PRODUCT if carry is not None else L.GX_AGG_SUM, result=res)
+    p.filter(filt, lo, hi)
+    if carry is not None:
+        p.carry(carry)
+    p.value(value)
+    p.launch()
+    api.scan_check()
+    return int(res.item())
+
+
+@pytest.mark.parametrize("bits", [1, 2, 7, 8, 9, 15, 16, 17, 24, 25, 31, 32])
+@pytest.mark.parametrize("n", [1, 3, 1023, 1025, 2049, 40_001, 100_003])
+def test_packed_widths(cuda, bits, n):
+    r = np.random.default_rng(bits * 1000 + n)
+    lo = -(1 << (bits - 1))
+    v = r.integers(lo, lo + (1 << bits), n, dtype=np.int64)
+    w = r.integers(0, 1000, n)
+    cv, cw = _col(v, "cascaded"), _col(w, "none")
+    a, b = np.quantile(v, [0.2, 0.8]).astype(np.int64)
+    m = (v >= a) & (v <= b)
+    assert _sum(cuda, cv, int(a), int(b), cw) == int(w[m].sum())
+    assert _sum(cuda, cw, 100, 800, cv) == int(v[(w >= 100) & (w <= 800)].sum())
+
+
+@pytest.mark.parametrize("run", [300, 700, 1500])
+@pytest.mark.parametrize("step", [1, 1000])
+def test_few_runs(cuda, run, step):
+    n = 90_011
+    r = np.random.default_rng(run)
+    v = np.repeat(np.arange(n // run + 1) * step - 5, run)[:n]
+    w, x = r.integers(-500, 500, n), r.integers(0, 50, n)
+    for codec in ("cascaded", "lz4"):
+        cv, cw, cx = _col(v, "cascaded"), _col(w, codec), _col(x, codec)
+        a, b = int(v[n // 5]), int(v[n // 2])
+        m = (v >= a) & (v <= b)
+        assert _sum(cuda, cv, a, b, cw, cx) == int((w[m] * x[m]).sum())
+
+
+@pytest.mark.parametrize("layout", ["linear", "bucket", "dense"])
+@pytest.mark.parametrize("entries,cap", [(5, 5), (1000, 513), (4095, 2048)])
+def test_chains_and_group_overflow(cuda, layout, entries, cap):
+    # tables filled past their nominal load (long chains), probed with keys half
+    # of which are absent; up to 4095 groups for 512 shared slots; negative values
+    n = 120_007
+    r = np.random.default_rng(entries)
+    keys = np.arange(1, entries + 1, dtype=np.int32) * 3
+    pay = r.permutation(entries).astype(np.int32)
+    ht = api.HashMap(cap, layout)
+    kd, pd = cuda.from_numpy(keys).cuda(), cuda.from_numpy(pay).cuda()
+    ht.build(kd, pd)
+    k = r.integers(0, entries + 2, n) * 3 - r.integers(0, 2, n)
+    val = r.integers(-2_000_000_000, 2_000_000_000, n)
+    date = np.sort(r.integers(0, 4, n))
+    fact = {c: _col(x, "cascaded" if c == "d" else "lz4") for c, x in (("k", k), ("v", val), ("d", date))}
+    agg = api.HashAggregate(entries * 4)
+    p = api.ScanPlan(agg=L.GX_AGG_SUM, groupby=agg)
+    p.probe(fact["k"], ht, 0, entries).group(fact["d"], 0, 4).value(fact["v"])
+    p.launch()
+    api.scan_check()
+    look = np.full(entries * 3 + 10, -1, np.int64)
+    look[keys] = pay
+    d = look[np.maximum(k, 0)]
+    d[k < 0] = -1
+    m = d >= 0
+    want = np.zeros(entries * 4, np.int64)
+    np.add.at(want, d[m] * 4 + date[m], val[m])
+    seen = np.unique(d[m] * 4 + date[m])
+    assert agg.read() == {int(g): int(want[g]) for g in seen}

@@ -463,9 +463,18 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
             } else {
                 used = casc_encode_block(vals + r0, rows, rle, delta, bp, buf, &col->seg[(size_t)2 * S * s]);
                 for (uint32_t p = 0; p * kCascPageRows < rows; ++p) {
+                    if (!all_simple.load(std::memory_order_relaxed)) break;
+                    const uint8_t* pg = buf.data() + start + col->seg[(size_t)2 * S * s + 2 * p];
                     casc_hdr h;
-                    std::memcpy(&h, buf.data() + start + col->seg[(size_t)2 * S * s + 2 * p], sizeof(h));
-                    if (!casc_page_simple(h.flags, h.n_runs, h.val_bits, h.val_base)) all_simple = false;
+                    std::memcpy(&h, pg, sizeof(h));
+                    bool two = true;
+                    if ((h.flags & CASC_RLE) && h.n_runs <= kCascFewRuns) {
+                        uint32_t end[kCascFewRuns], e = 0;
+                        for (uint32_t k = 0; k < h.n_runs; ++k)
+                            end[k] = e += unpack_bits((const uint32_t*)(pg + h.lens_off), k, h.len_bits) + h.len_base;
+                        two = casc_two_per_tile(h.n_runs, [&](uint32_t k) { return end[k]; });
+                    }
+                    if (!casc_page_simple(h.flags, h.n_runs, h.val_bits, h.val_base, two)) all_simple = false;
                 }
             }
             buf.resize((buf.size() + kPayloadAlign - 1) & ~(size_t)(kPayloadAlign - 1), 0);

@@ -38,11 +38,13 @@ namespace {
 
 constexpr uint32_t kGencNT = 256;
 
+constexpr uint32_t kPlanTwoPerTile = 1u << 8;  // few runs, at most two on a tile (casc_two_per_tile)
+
 // The chosen encoding of one cascaded page (pass 1 -> host -> pass 2).
 struct PagePlan {
     uint32_t bytes;   // page bytes (a multiple of 16)
     uint32_t n;       // values in the value stream (rows, or runs with RLE)
-    uint32_t flags;   // CASC_RLE | CASC_DELTA
+    uint32_t flags;   // CASC_RLE | CASC_DELTA, and kPlanTwoPerTile
     uint32_t vbits, lbits;
     int32_t vbase;    // frame of reference of the value stream
     uint32_t lbase;   // frame of reference of the run lengths
@@ -228,6 +230,8 @@ __global__ void __launch_bounds__(kGencNT) genc_plan_kernel(const GencParams P) 
             }
         }
     }
+    if ((best.flags & CASC_RLE) && nr <= kCascFewRuns && casc_two_per_tile(nr, [&](uint32_t k) { return start[k + 1]; }))
+        best.flags |= kPlanTwoPerTile;
     P.plans[(size_t)s * P.pages + p] = best;
 }
 
@@ -289,7 +293,7 @@ __global__ void __launch_bounds__(kGencNT) genc_write_kernel(const GencParams P)
         uint32_t* h = (uint32_t*)pg;
         h[0] = n;
         h[1] = pl.n;
-        h[2] = pl.flags | (pl.vbits << 8) | ((rle ? pl.lbits : 0u) << 16);
+        h[2] = (pl.flags & (CASC_RLE | CASC_DELTA)) | (pl.vbits << 8) | ((rle ? pl.lbits : 0u) << 16);
         h[3] = (uint32_t)pl.first;
         h[4] = (uint32_t)pl.vbase;
         h[5] = rle ? pl.lbase : 0u;
@@ -487,7 +491,8 @@ extern "C" gx_status gx_column_encode_device(const int32_t* values_dev, uint64_t
                 for (uint32_t p = 0; p < n_pages; ++p) {
                     const PagePlan& pl = plans[(size_t)sl * pages + p];
                     const uint32_t b = pl.bytes;
-                    if (!casc_page_simple(pl.flags, pl.n, pl.vbits, pl.vbase)) simple = false;
+                    if (!casc_page_simple(pl.flags, pl.n, pl.vbits, pl.vbase, (pl.flags & kPlanTwoPerTile) != 0))
+                        simple = false;
                     po[p] = off;
                     col->seg[(size_t)2 * S * sl + 2 * p] = off;
                     col->seg[(size_t)2 * S * sl + 2 * p + 1] = b;

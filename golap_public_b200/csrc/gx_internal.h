@@ -76,7 +76,8 @@ constexpr uint32_t kCascMaxRuns = 2048;        // run tables of one decode (>= k
 constexpr uint32_t kCascPageLog2 = 11;
 constexpr uint32_t kCascPageRows = 1u << kCascPageLog2;  // rows of one cascaded page
 constexpr uint32_t kCascPageMaxRuns = 512;     // RLE pages hold at most this many runs
-constexpr uint32_t kCascFewRuns = 8;           // RLE pages of at most this many runs are scanned without a decode
+constexpr uint32_t kCascFewRuns = 8;           // RLE pages of at most this many runs may be scanned without a decode
+constexpr uint32_t kCascTileRows = 1024;       // ... when no aligned tile of this many rows holds more than two runs
 constexpr uint32_t kCascMaxPages = kMaxRowsPerBlock / kCascPageRows;
 constexpr uint32_t kStageBytes = 66048;        // shared staging buffer for one compressed block
 constexpr uint32_t kPayloadAlign = 16;
@@ -102,9 +103,11 @@ struct casc_hdr {
 static_assert(sizeof(casc_hdr) == 32, "casc_hdr layout");
 
 // A page the warp-tile scan evaluates from its own bytes: bit-packed values
-// without RLE or DELTA, one value, or a few runs.
-GX_HOSTDEV inline bool casc_page_simple(uint32_t flags, uint32_t n_runs, uint32_t val_bits, int32_t val_base) {
-    if (flags & CASC_RLE) return n_runs <= kCascFewRuns;
+// without RLE or DELTA, one value, or few runs of which no tile holds more
+// than two (two_per_tile, for RLE pages of at most kCascFewRuns runs).
+GX_HOSTDEV inline bool casc_page_simple(uint32_t flags, uint32_t n_runs, uint32_t val_bits, int32_t val_base,
+                                        bool two_per_tile) {
+    if (flags & CASC_RLE) return n_runs <= kCascFewRuns && two_per_tile;
     return !(flags & CASC_DELTA) || (val_bits == 0 && val_base == 0);
 }
 
@@ -145,6 +148,15 @@ GX_HOSTDEV inline uint32_t unpack_bits(const uint32_t* words, uint32_t i, uint32
     uint64_t two = (uint64_t)words[wi] | ((uint64_t)words[wi + 1] << 32);
     uint64_t mask = (w == 32) ? 0xFFFFFFFFull : ((1ull << w) - 1);
     return (uint32_t)((two >> sh) & mask);
+}
+
+// Whether no aligned kCascTileRows-row tile of a page holds more than two of
+// its n runs; end(k) = row after run k.
+template <class F>
+GX_HOSTDEV inline bool casc_two_per_tile(uint32_t n, F end) {
+    for (uint32_t k = 1; k + 1 < n; ++k)  // run k inside one tile, with a neighbour on both sides there
+        if (end(k - 1) % kCascTileRows != 0 && end(k - 1) / kCascTileRows == end(k) / kCascTileRows) return false;
+    return true;
 }
 
 // Join/group table hashing: the public definitions in include/gx_hash.h.

@@ -23,7 +23,7 @@
 //     runs too) and writes to the warp's records in shared memory how the
 //     column is read -- direct (raw rows or a 16-byte aligned LZ4 literal run:
 //     the evaluator loads the rows from HBM itself), from the page's own bytes
-//     (bit-packed values, two runs, a few runs), constant (one value on the
+//     (bit-packed values, two runs), constant (one value on the
 //     tile), or decoded by the warp into its buffer (LZ4 ranges with matches:
 //     groups of lanes per segment; other cascaded pages: run windows of 32
 //     runs, one per lane).  The next round's directory lines are prefetched,
@@ -76,6 +76,7 @@ constexpr uint32_t kWsMaxChunkWords = 1024;     // chunk keep bits of one launch
 constexpr uint32_t kWsHead = 32 * 8 + 8 * 8 + 2 * GX_MAX_STEPS + 32 + 4;
 constexpr uint32_t kWsQueueWords = (kWsBatch + 32) * 3;  // grouped plans: the warp's WsQueue, before its decode buffers
 static_assert(kWsHead % 4 == 0, "decode buffers start 16-byte aligned");
+static_assert(kWsTile == kCascTileRows, "simple cascaded pages are simple for the scan's tiles");
 static_assert(kWsTile <= kCascPageRows && kCascPageRows % kWsTile == 0, "a warp tile lies in one cascaded page");
 
 struct WsParams {
@@ -103,11 +104,10 @@ struct WsParams {
 // Cascaded pages that the evaluator reads from their own bytes, without a
 // decode: kWmPack, bit-packed values without RLE or DELTA (four values of a
 // lane from up to five words); kWmRuns2, a tile of a few-run page covered by
-// two runs (value cval on tile rows [0, aux0), value aux1 from there);
-// kWmRuns, a tile of more runs of such a page.
+// two runs (value cval on tile rows [0, aux0), value aux1 from there).
 // kWmRows: in shared memory, after the warp's decode.
 enum : uint32_t {
-    kWmDirect = 0, kWmConst = 1, kWmLz4 = 2, kWmCasc = 3, kWmBad = 4, kWmRuns2 = 5, kWmRows = 6, kWmPack = 7, kWmRuns = 8
+    kWmDirect = 0, kWmConst = 1, kWmLz4 = 2, kWmCasc = 3, kWmBad = 4, kWmRuns2 = 5, kWmRows = 6, kWmPack = 7
 };
 
 // Inclusive warp scan (wrapping uint32 sum).
@@ -330,7 +330,7 @@ struct __align__(16) WsTile {
     uint32_t pad;
 };
 constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
-constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a probe's constant or two-run one
+constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a probe's that is not packed
 static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
 
 // How one column of one tile is read.
@@ -340,7 +340,7 @@ struct __align__(16) WsCol {
     int32_t cval;         // kWmConst: the value; kWmRuns2: the first run's; kWmPack: the frame of reference
     uint32_t aux0, aux1;  // LZ4: [lo, hi) in the block; cascaded: page bytes, page rows; kWmRuns2: the first
                           // run's end, the second's value; kWmPack: bits per value
-    uint32_t bytes;       // LZ4: the block's compressed bytes; kWmPack, kWmRuns: the tile's first row in the page
+    uint32_t bytes;       // LZ4: the block's compressed bytes; kWmPack: the tile's first row in the page
     uint32_t pad;
 };
 static_assert(sizeof(WsCol) == 32, "column records of 8 words");
@@ -500,13 +500,6 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
                                 break;
                             }
                         }
-                        if (C.mode != kWmConst && C.mode != kWmRuns2) {
-                            // more runs on the tile: read run by run, if they add up to the page
-                            uint32_t sum = 0;
-                            for (uint32_t k = 0; k < h.n_runs; ++k) sum += unpack_bits(lw, k, h.len_bits) + h.len_base;
-                            C.mode = sum == C.aux1 ? kWmRuns : kWmBad;
-                            C.bytes = h0;
-                        }
                     }
                 }
             }
@@ -588,7 +581,7 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
         const ShStep& st = Q.steps[s];
         const WsCol& c = cols[(q << cl) + st.col];
         isc = c.mode == kWmConst;
-        mixed = c.mode != kWmDirect && !((isc || c.mode == kWmRuns2) && (st.flags & GX_STEP_PROBE));
+        mixed = c.mode != kWmDirect && (c.mode == kWmPack || !(st.flags & GX_STEP_PROBE));
         if (isc) {
             const int32_t v = c.cval;
             int32_t pp = v;
@@ -740,28 +733,6 @@ __device__ __forceinline__ uint4 ws_unpack4(const uint32_t* words, uint32_t i, u
     return make_uint4((a0 & mask) + base, at(w), at(2 * w), at(3 * w));
 }
 
-// Rows i .. i + 3 of a few-run page, run by run (the decision has checked the
-// header and that the runs add up to the page).
-__device__ __noinline__ uint4 ws_runs4(const uint8_t* pg, uint32_t i) {
-    const casc_hdr h = casc_load_header(pg);
-    const bool delta = (h.flags & CASC_DELTA) != 0;
-    const uint32_t* vw = (const uint32_t*)(pg + h.vals_off);
-    const uint32_t* lw = (const uint32_t*)(pg + h.lens_off);
-    uint32_t start = 0, val = delta ? (uint32_t)h.first : 0u;
-    uint4 v = make_uint4(0, 0, 0, 0);
-#pragma unroll 1
-    for (uint32_t k = 0; k < h.n_runs; ++k) {
-        const uint32_t e = (delta && k == 0) ? 0u : unpack_bits(vw, k, h.val_bits) + (uint32_t)h.val_base;
-        val = delta ? val + e : e;
-        if (i >= start) v.x = val;
-        if (i + 1 >= start) v.y = val;
-        if (i + 2 >= start) v.z = val;
-        if (i + 3 >= start) v.w = val;
-        start += unpack_bits(lw, k, h.len_bits) + h.len_base;
-    }
-    return v;
-}
-
 template <uint32_t R>
 __device__ __forceinline__ void ws_put(uint32_t (&w)[R], uint32_t h, const uint4& x) {
     w[4 * h] = x.x;
@@ -784,7 +755,6 @@ __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
     const uint32_t v0 = (uint32_t)d.cval;
     if (mode == kWmConst) return make_uint4(v0, v0, v0, v0);
     if (mode == kWmRuns2) return ws_runs2(d, row);
-    if (mode == kWmRuns) return ws_runs4(d.src, d.bytes + row);
     return *(const uint4*)(d.src + 4 * row);  // kWmRows
 }
 
@@ -795,9 +765,9 @@ __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
 // is used and unrolls its steps: up to the last probe step by step, the
 // filters after it and the aggregate row by row, where a row's mask is a
 // predicate.  The run-time form (SIG 0) loads a column at its step.  FLAT:
-// [a, b) is whole batches and every column is direct or a probe's constant or
-// two-run one (a sorted date), so that a batch's loads are unconditional and
-// all in flight together.  Steps over constant columns were decided by
+// [a, b) is whole batches and every column is direct, or a probe's and constant,
+// of two runs or decoded (a sorted date), so that a batch's loads are
+// unconditional and all in flight together.  Steps over constant columns were decided by
 // ws_const_steps.
 // Returns the scalar part; grouped sums go to the CTA's group table through
 // the warp's queue.
@@ -850,8 +820,11 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
                     asm("" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w));
                     if (FLAT) {
                         const WsCol& d = cols[Q.steps[s].col];
-                        if (((SIG >> (7 + 4 * s)) & kWkP) && !skip && d.mode == kWmRuns2)
+                        const bool probe = ((SIG >> (7 + 4 * s)) & kWkP) != 0;
+                        if (probe && !skip && d.mode == kWmRuns2)
                             x = ws_runs2(d, row + kWsBatch * h);
+                        else if (probe && !skip && d.mode == kWmRows)
+                            x = *(const uint4*)(d.src + 4 * (row + kWsBatch * h));
                         else if (!skip)
                             x = ws_ld_rows(src[s] + kWsBatch * 4 * h);
                     } else if (cols[Q.steps[s].col].mode == kWmDirect && row + kWsBatch * h < b) {

@@ -1816,6 +1816,7 @@ static gx_status ensure_kernel_attrs() {
     if (!st) st = allow_smem(warp_scan_kernel<kSigQ2>, kWsMaxDynSmem);
     if (!st) st = allow_smem(warp_scan_kernel<kSigQ3>, kWsMaxDynSmem);
     if (!st) st = allow_smem(warp_scan_kernel<kSigQ4>, kWsMaxDynSmem);
+    if (!st) st = allow_smem(warp_scan_kernel<kSigGroup>, kWsMaxDynSmem);
     if (st) return st;
     attr_set[dev] = true;
     return GX_OK;
@@ -2285,6 +2286,7 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     else if (sig == kSigQ2) kern = warp_scan_kernel<kSigQ2>;
     else if (sig == kSigQ3) kern = warp_scan_kernel<kSigQ3>;
     else if (sig == kSigQ4) kern = warp_scan_kernel<kSigQ4>;
+    else if (sig == kSigGroup) kern = warp_scan_kernel<kSigGroup>;
     P.warp_words = kWsHead + (P.grouped_tab ? kWsQueueWords : 0u) + areas * kWsTile;
     const size_t smem = 4ull * (2ull * P.chunk_words + (size_t)P.warp_words * kWsWarps +
                                 (P.grouped_tab ? 3ull * kWsGroupSlots : 0ull));

@@ -330,7 +330,7 @@ struct __align__(16) WsTile {
     uint32_t pad;
 };
 constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
-constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a probe's that is not packed
+constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a loose step's that is not packed
 static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
 
 // How one column of one tile is read.
@@ -565,6 +565,13 @@ __device__ __forceinline__ bool ws_probe1(const ShStep& st, uint64_t hdr, int32_
     return true;
 }
 
+// Steps whose column need not be direct in the flat evaluator (constant, of
+// two runs or decoded will do): probes and the first step, when they neither
+// carry nor are the last.
+__device__ constexpr bool ws_loose_step(uint32_t s, uint32_t n_steps, bool probe, bool carry) {
+    return (probe || s == 0) && !carry && s + 1 < n_steps;
+}
+
 // The steps over columns that hold one value on their tile, decided once per
 // tile and for all tiles of the round together (their probes are one chain of
 // loads): lane (q << cl) + s decides step s of tile q, leaves its group-key
@@ -581,7 +588,9 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
         const ShStep& st = Q.steps[s];
         const WsCol& c = cols[(q << cl) + st.col];
         isc = c.mode == kWmConst;
-        mixed = c.mode != kWmDirect && (c.mode == kWmPack || !(st.flags & GX_STEP_PROBE));
+        mixed = c.mode != kWmDirect &&
+                (c.mode == kWmPack || !ws_loose_step(s, Q.n_steps, (st.flags & GX_STEP_PROBE) != 0,
+                                                     (st.flags & GX_STEP_CARRY) != 0));
         if (isc) {
             const int32_t v = c.cval;
             int32_t pp = v;
@@ -629,6 +638,8 @@ constexpr uint32_t kSigQ3 = ws_sig(4, GX_AGG_SUM, true, kWkP | kWkD, kWkP | kWkD
 // pipeline_q2: part probe (brand digit), supplier probe, date probe (year digit), revenue grouped
 constexpr uint32_t kSigQ2 = ws_sig(4, GX_AGG_SUM, true, kWkP | kWkD, kWkP, kWkP | kWkD, 0);
 // pipeline_q4: customer (nation digit), supplier, date (year digit), part probes, supplycost carried, profit grouped
+// a group-by of one column over a range of another (dates): value grouped by a digit
+constexpr uint32_t kSigGroup = ws_sig(3, GX_AGG_SUM, true, kWkF, kWkD, 0);
 constexpr uint32_t kSigQ4 = ws_sig(6, GX_AGG_SUM_DIFF, true, kWkP | kWkD, kWkP, kWkP | kWkD, kWkP, kWkC, 0);
 
 // A join-table probe of R rows per lane (R = 4 per row group): rows whose bit
@@ -688,9 +699,10 @@ __device__ __forceinline__ uint32_t ws_probe_rows(const ShStep& st, uint64_t hdr
     return m & ~u;
 }
 
-// The last probe step of a signature, plus one (0: none).
+// The steps of a signature that run step by step: up to the last probe, and
+// the first one (often the sort key's filter, decided for the whole tile).
 constexpr uint32_t ws_probes_end(uint32_t sig) {
-    uint32_t e = 0;
+    uint32_t e = 1;
     for (uint32_t s = 0; s < (sig & 7); ++s)
         if ((sig >> (7 + 4 * s)) & kWkP) e = s + 1;
     return e;
@@ -765,9 +777,9 @@ __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
 // is used and unrolls its steps: up to the last probe step by step, the
 // filters after it and the aggregate row by row, where a row's mask is a
 // predicate.  The run-time form (SIG 0) loads a column at its step.  FLAT:
-// [a, b) is whole batches and every column is direct, or a probe's and constant,
-// of two runs or decoded (a sorted date), so that a batch's loads are
-// unconditional and all in flight together.  Steps over constant columns were decided by
+// [a, b) is whole batches and every column is direct or a loose step's that is
+// not packed (a sorted date), so that a batch's loads are unconditional and all
+// in flight together.  Steps over constant columns were decided by
 // ws_const_steps.
 // Returns the scalar part; grouped sums go to the CTA's group table through
 // the warp's queue.
@@ -813,17 +825,18 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
             // wanted row ends at most 12 bytes after its block, inside the payload)
 #pragma unroll
             for (uint32_t s = 0; s < NS; ++s) {
-                const bool skip = ((SIG >> (7 + 4 * s)) & kWkP) && ((cst >> s) & 1u);
+                const uint32_t K = (SIG >> (7 + 4 * s)) & 15u;
+                const bool loose = ws_loose_step(s, NS, (K & kWkP) != 0, (K & kWkC) != 0);
+                const bool skip = loose && ((cst >> s) & 1u);
 #pragma unroll
                 for (uint32_t h = 0; h < H; ++h) {
                     uint4 x;
                     asm("" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w));
                     if (FLAT) {
                         const WsCol& d = cols[Q.steps[s].col];
-                        const bool probe = ((SIG >> (7 + 4 * s)) & kWkP) != 0;
-                        if (probe && !skip && d.mode == kWmRuns2)
+                        if (loose && !skip && d.mode == kWmRuns2)
                             x = ws_runs2(d, row + kWsBatch * h);
-                        else if (probe && !skip && d.mode == kWmRows)
+                        else if (loose && !skip && d.mode == kWmRows)
                             x = *(const uint4*)(d.src + 4 * (row + kWsBatch * h));
                         else if (!skip)
                             x = ws_ld_rows(src[s] + kWsBatch * 4 * h);
@@ -1002,10 +1015,12 @@ __device__ __noinline__ int64_t ws_eval_any(const ShQuery& Q, const WsCol* cols,
 // their columns in registers) keep 96 registers: five CTAs, 20 warps, scan Q1
 // over 60M rows in 132 us where four take 165 us (too few loads in flight) and
 // six 150 us (spills).  Grouped ones (one row group, probes) take six: the
-// 200M-row star join 2.17 ms, 2.26 with five, 2.35 with seven.  Run-time plans
-// wait on group-table adds and take eight (778 us against 909 us with five,
-// 30M rows into 1.4M groups).
-constexpr int ws_ctas(uint32_t sig) { return sig == 0 ? 8 : ((sig >> 6) & 1) ? 6 : 5; }
+// 200M-row star join 2.17 ms, 2.26 with five, 2.35 with seven; more shared
+// memory costs them L1, which holds their reads in flight: 2048 group slots
+// instead of 512, 4.2 ms).  The group-by without joins and run-time plans wait
+// on group-table adds and take eight (30M rows into 1.4M groups: 585 us, 674
+// with six; as a run-time plan 782).
+constexpr int ws_ctas(uint32_t sig) { return sig == 0 || sig == kSigGroup ? 8 : ((sig >> 6) & 1) ? 6 : 5; }
 
 template <uint32_t SIG>
 __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __grid_constant__ WsParams P) {

@@ -92,3 +92,30 @@ def test_chains_and_group_overflow(cuda, layout, entries, cap):
     np.add.at(want, d[m] * 4 + date[m], val[m])
     seen = np.unique(d[m] * 4 + date[m])
     assert agg.read() == {int(g): int(want[g]) for g in seen}
+
+
+@pytest.mark.parametrize("n", [1, 1025, 300_001])
+@pytest.mark.parametrize("date", ["sorted", "few_runs", "random"])
+def test_group_by_of_a_range(cuda, n, date):
+    # the group-by template (filter, group column, value): constant, two-run,
+    # decoded and packed filter columns, an empty range, a digit out of range
+    r = np.random.default_rng(n)
+    d = {"sorted": np.sort(r.integers(0, 20, n)), "few_runs": np.sort(r.integers(0, n // 300 + 1, n)),
+         "random": r.integers(0, 1000, n)}[date]
+    k, v = r.integers(7, 2007, n), r.integers(-10**9, 10**9, n)
+    cd, ck, cv = _col(d, "cascaded"), _col(k, "lz4"), _col(v, "none")
+    for lo, hi in ((int(np.quantile(d, 0.1)), int(np.quantile(d, 0.9))), (5, 4)):
+        agg = api.HashAggregate(2000)
+        api.ScanPlan(agg=L.GX_AGG_SUM, groupby=agg).filter(cd, lo, hi).group(ck, 7, 2000).value(cv).launch()
+        api.scan_check()
+        m = (d >= lo) & (d <= hi)
+        want = np.zeros(2000, np.int64)
+        np.add.at(want, k[m] - 7, v[m])
+        assert agg.read() == {int(g): int(want[g]) for g in np.unique(k[m] - 7)}
+    agg = api.HashAggregate(2000)
+    api.ScanPlan(agg=L.GX_AGG_SUM, groupby=agg).filter(cd, 0, 10**6).group(ck, 8, 2000).value(cv).launch()
+    if (k == 7).any():
+        with pytest.raises(api.L.GxError):
+            api.scan_check()
+    else:
+        api.scan_check()

@@ -412,6 +412,7 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
     if (threads == 0) threads = std::max(1u, std::thread::hardware_concurrency());
     threads = std::min<uint32_t>(threads, std::max<uint32_t>(1, col->n_slots));
     std::vector<std::vector<uint8_t>> bufs(threads);
+    std::atomic<uint64_t> seqs{0};
     std::atomic<bool> overflow{false}, all_simple{codec == GX_CODEC_CASCADED};
     std::vector<std::vector<uint64_t>> local_off(threads);
     auto work = [&](uint32_t t) {
@@ -445,12 +446,13 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
                 buf.insert(buf.end(), (const uint8_t*)(vals + r0), (const uint8_t*)(vals + r0 + rows));
                 used = (size_t)rows * 4;
             } else if (codec == GX_CODEC_LZ4) {
-                uint32_t tmp_seg[2 * kMaxSegments];
+                uint32_t tmp_seg[2 * kMaxSegments], n_seq = 0;
                 lz4_tmp.clear();
                 used = min_match ? lz4_encode_block(vals + r0, rows, S, rows_per_block / S, min_match, depth, lz4_tmp,
-                                                    tmp_seg, nullptr)
+                                                    tmp_seg, &n_seq)
                                  : lz4_encode_block_auto(vals + r0, rows, S, rows_per_block / S, depth, lz4_tmp,
                                                          tmp_seg);
+                seqs += n_seq;
                 if (used + 16 > kStageBytes) overflow = true;  // cannot happen for <= 16384 int32 rows
                 if (S > 1) std::memcpy(&col->seg[(size_t)2 * S * s], tmp_seg, 8 * S);
                 // place the block so that its first literal byte is 16-byte aligned
@@ -489,6 +491,7 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
     work(0);
     for (auto& th : pool) th.join();
     col->casc_simple = all_simple;
+    col->lz4_seqs = seqs;
     if (overflow) return set_error(GX_ERR_INVALID, "an LZ4 block exceeds the %u-byte staging buffer", kStageBytes);
     // the per-thread buffers in thread order, each copied by its own thread
     std::vector<uint64_t> shift(threads + 1, 0);

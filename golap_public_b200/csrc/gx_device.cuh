@@ -139,81 +139,246 @@ __device__ __forceinline__ bool lz4_len_ext(const uint32_t* __restrict__ A, uint
     }
 }
 
-// Decodes one segment of a segmented LZ4 block with a group of G lanes
-// (G a power of two <= 32, the group's lanes adjacent in one warp; gmask =
-// the group's lanes, gl = this lane's index in the group).  Every lane of the
-// group parses the same sequence headers (broadcast shared loads), so the
-// group stays converged; literal runs and matches are copied G words per
-// step.  A match's words are all computed from output before the match:
-// out[k + i] = out[k - offw + (i mod offw)] (LZ4 overlap semantics), so one
-// __syncwarp before each match orders it after every earlier write of the
-// group.  Same stream contract as the per-lane decoder: A = staged words
-// from byte wbase, [lo, hi) the tile's compressed range, K output words.
-// Returns 0 or kErrCorrupt (identical on every lane of the group).
-__device__ __forceinline__ int lz4_seg_group(const uint32_t* __restrict__ A, uint32_t wbase, uint32_t lo,
-                                             uint32_t hi, uint32_t block_end, uint32_t comp_pos, uint32_t info,
-                                             uint32_t K, uint32_t* __restrict__ out, uint32_t gl, uint32_t G,
-                                             uint32_t gmask) {
-    if (comp_pos < lo || comp_pos > hi) return kErrCorrupt;
+// Decodes one segment of a segmented LZ4 block per group of G lanes (G a power
+// of two <= 32, a group's lanes adjacent; gl = this lane's index in it), the
+// groups of a warp in step: one sequence each per round.  Called by whole
+// warps; lanes of a group without a segment pass active = false.  Every lane
+// of a group parses the same sequence headers (broadcast loads); literal runs
+// and matches are copied G words per step.  A match's words are all computed
+// from output before the match: out[k + i] = out[k - offw + (i mod offw)] (LZ4
+// overlap semantics), so the barrier before each match orders it after every
+// earlier write of the group.  A = the words from byte wbase (staged, or in
+// place), [lo, hi) the tile's compressed range, K output words.  Returns 0 or
+// kErrCorrupt (the same for every lane of a group).
+// What bounds it: the chain of dependent instructions of a sequence (100 or
+// so, 6 to 8 cycles each with few warps resident), of which a segment of small
+// integers has nearly one per row.  A round of short sequences therefore reads
+// token, offset and one literal extension byte from one unaligned word and
+// fetches the next token before the copy, and the groups stay in step (their
+// own loops drifted apart and ran one after another).  Q1 over 10M rows of such
+// columns 665 -> 570 us, decoding 24M discount rows 353 -> 330; a column known
+// to hold many short sequences takes lz4_seg_lane in the scan.
+__device__ __forceinline__ int lz4_seg_step(const uint32_t* __restrict__ A, uint32_t wbase, uint32_t lo, uint32_t hi,
+                                            uint32_t block_end, uint32_t comp_pos, uint32_t info, uint32_t K,
+                                            uint32_t* __restrict__ out, uint32_t gl, uint32_t G, bool active) {
     uint32_t pos = comp_pos, k = 0, litw = 0, mnib = 0;
-    bool tok_next = true;
-    if (info & 16u) {  // the segment starts inside a sequence
-        const uint32_t lit = info >> 5;
-        if (lit & 3u) return kErrCorrupt;
-        litw = lit >> 2;
+    bool ok = comp_pos >= lo && comp_pos <= hi, run = active && ok;
+    bool tok = true;  // the next thing is a token
+    if (run && (info & 16u)) {  // the segment starts inside a sequence
+        ok = ((info >> 5) & 3u) == 0;
+        litw = info >> 7;
         mnib = info & 15u;
-        tok_next = false;
+        tok = false;
     }
-    while (true) {
-        if (tok_next) {
-            if (k >= K) break;
-            if (pos >= hi) return kErrCorrupt;
-            const uint32_t x = fetch4(A, pos - wbase);
-            uint32_t lit = (x >> 4) & 15u;
-            mnib = x & 15u;
-            ++pos;
-            if (lit == 15 && !lz4_len_ext(A, wbase, pos, hi, lit)) return kErrCorrupt;
-            if (lit & 3u) return kErrCorrupt;
-            litw = lit >> 2;
+    run = run && ok && (k < K || !tok);
+    if (!run) pos = lo;  // lanes without work read some word of the range
+    uint32_t x = fetch4(A, pos - wbase);
+    while (__any_sync(0xFFFFFFFFu, run)) {
+        const uint32_t tl = (x >> 4) & 15u, tm = x & 15u;
+        const bool ext = tl == 15u && ((x >> 8) & 255u) == 255u;  // longer literals than one extension byte gives
+        if (!__any_sync(0xFFFFFFFFu, run && (!tok || ext || tm == 15u))) {
+            // ---- a round of short sequences: at most 67 literal words, at most 4 match words
+            const uint32_t lit = tl == 15u ? 15u + ((x >> 8) & 255u) : tl, q0 = pos + (tl == 15u ? 2u : 1u);
+            const uint32_t lw = lit >> 2, n = min(lw, K - k), q = q0 - wbase, kk = k + n;
+            const bool more = lw < K - k;  // the segment goes on with the match
+            uint32_t off = x >> 8;
+            bool good = (lit & 3u) == 0 && q0 + 4 * n <= hi;
+            if (__any_sync(0xFFFFFFFFu, run && lit)) {
+                if (run && good)
+                    for (uint32_t i = gl; i < n; i += G) out[k + i] = fetch4(A, q + 4 * i);
+                if (lit && run && good && more) off = fetch4(A, q + lit);
+            }
+            off &= 0xFFFFu;
+            const uint32_t offw = off >> 2, mw = more ? (tm >> 2) + 1 : 0u;
+            const uint32_t p1 = q0 + lit;
+            if (more)
+                good = good && p1 != block_end && p1 + 2 <= hi && ((off | tm) & 3u) == 0 && offw - 1u < kk && mw <= K - kk;
+            if (run && !good) ok = run = false;
+            __syncwarp();
+            const uint32_t nx = run && more ? fetch4(A, p1 + 2 - wbase) : x;  // the next token, ahead of the copy
+            if (run)
+                for (uint32_t i = gl; i < mw; i += G) {
+                    uint32_t r = i;
+                    if (offw < 4) r = offw == 1 ? 0u : offw == 2 ? (i & 1u) : (i == 3 ? 0u : i);
+                    out[kk + i] = out[kk - offw + r];
+                }
+            if (run) {
+                k = kk + mw;
+                pos = p1 + 2;
+                x = nx;
+            }
+            run = run && more && k < K;
+            __syncwarp();
+            continue;
         }
-        const uint32_t n = min(litw, K - k);
-        if ((uint64_t)pos + 4ull * n > hi) return kErrCorrupt;
+        // ---- the general round
+        if (run && tok) {
+            ok = pos < hi;
+            if (ok) {
+                uint32_t lit = tl;
+                mnib = tm;
+                ++pos;
+                if (lit == 15) ok = lz4_len_ext(A, wbase, pos, hi, lit);
+                ok = ok && (lit & 3u) == 0;
+                litw = lit >> 2;
+            }
+            run = ok;
+        }
+        uint32_t n = run ? min(litw, K - k) : 0u;
+        if (run && (uint64_t)pos + 4ull * n > hi) {
+            ok = run = false;
+            n = 0;
+        }
         {
             const uint32_t r = pos - wbase, w = r >> 2, sh = (r & 3u) * 8;
             for (uint32_t i = gl; i < n; i += G) out[k + i] = __funnelshift_r(A[w + i], A[w + i + 1], sh);
         }
         k += n;
         pos += 4 * n;
-        if (k >= K) break;  // the segment ends inside or right after the literals
-        // literals done: the block may end here (then the segment is short)
-        if (pos == block_end || (uint64_t)pos + 2 > hi) return kErrCorrupt;
-        const uint32_t off = fetch4(A, pos - wbase) & 0xFFFFu;
-        pos += 2;
-        uint32_t ml = mnib + 4;
-        if (mnib == 15 && !lz4_len_ext(A, wbase, pos, hi, ml)) return kErrCorrupt;
-        if ((off & 3u) || (ml & 3u) || off == 0) return kErrCorrupt;
-        const uint32_t offw = off >> 2, mw = ml >> 2;
-        if (offw > k || mw > K - k) return kErrCorrupt;
-        __syncwarp(gmask);
-        const uint32_t* src = out + (k - offw);
-        if (offw >= mw) {
-            for (uint32_t i = gl; i < mw; i += G) out[k + i] = src[i];
-        } else if (offw == 1) {
-            const uint32_t v = src[0];
-            for (uint32_t i = gl; i < mw; i += G) out[k + i] = v;
-        } else {
-            uint32_t r = gl % offw;
-            const uint32_t step = G % offw;
-            for (uint32_t i = gl; i < mw; i += G) {
-                out[k + i] = src[r];
-                r += step;
-                if (r >= offw) r -= offw;
+        run = run && k < K;  // else the segment ends inside or right after the literals
+        // the match (the block may not end before it: then the segment is short)
+        uint32_t offw = 1, mw = 0;
+        if (run) {
+            ok = pos != block_end && (uint64_t)pos + 2 <= hi;
+            if (ok) {
+                const uint32_t off = fetch4(A, pos - wbase) & 0xFFFFu;
+                pos += 2;
+                uint32_t ml = mnib + 4;
+                if (mnib == 15) ok = lz4_len_ext(A, wbase, pos, hi, ml);
+                ok = ok && (off & 3u) == 0 && (ml & 3u) == 0 && off != 0;
+                offw = off >> 2;
+                mw = ml >> 2;
+                ok = ok && offw <= k && mw <= K - k;
+            }
+            run = ok;
+            if (!ok) mw = 0;
+        }
+        __syncwarp();
+        {
+            const bool wrap = offw < mw;
+            uint32_t r = gl, st = G;
+            if (wrap && offw != 1) {
+                r = gl % offw;
+                st = G % offw;
+            }
+            const uint32_t* src = out + (k - offw);
+            if (offw == 1) {
+                const uint32_t v = mw ? src[0] : 0u;
+                for (uint32_t i = gl; i < mw; i += G) out[k + i] = v;
+            } else {
+                for (uint32_t i = gl; i < mw; i += G) {
+                    out[k + i] = src[r];
+                    r += st;
+                    if (wrap && r >= offw) r -= offw;
+                }
             }
         }
         k += mw;
-        tok_next = true;
+        tok = true;
+        run = run && k < K;
+        if (run) x = fetch4(A, pos - wbase);
+        __syncwarp();
     }
-    return 0;
+    return active && !ok ? kErrCorrupt : 0;
+}
+
+// ---- one lane per segment, from staged bytes
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// 4 bytes at shared-memory address a, any alignment.
+__device__ __forceinline__ uint32_t lds32u(uint32_t a) {
+    const uint32_t b = a & ~3u;
+    return __funnelshift_r(lds32(b), lds32(b + 4), a * 8);  // (the shift counts modulo 32)
+}
+// Decodes one segment of a segmented LZ4 block per lane, two output words of a
+// sequence per round, for segments of many short sequences.  p = shared-memory address of
+// the byte at the segment's entry position, hi and block_end those of the ends
+// of the staged range and of the block; info and K as in lz4_seg_step; out =
+// shared-memory address of the segment's words (segments a multiple of four
+// words apart, not of 32: neighbouring lanes store to different banks).
+// Called by whole warps (active = false: no segment).  Returns false on a
+// corrupt stream.
+// Why: a sequence of small integers is a word or two long, so the work is the
+// parse of its header, whichever lanes are idle.  With a group of 4 lanes per
+// segment (lz4_seg_step) a warp parses 8 at a time, with one lane up to 32; a
+// header's token and offset are read at once (the offset's place follows from
+// the token), conditions are combined without branches, and literal and match
+// words take one path, so that the lanes stay together.  Length extensions of
+// more than two bytes cannot occur in a segment of at most 128 words.
+__device__ __forceinline__ bool lz4_seg_lane(uint32_t p, uint32_t hi, uint32_t block_end, uint32_t info, uint32_t K,
+                                             uint32_t out, bool active) {
+    uint32_t L = 0, M = 0;      // literal and match words left of the sequence
+    uint32_t lp = p, src = out; // where they are
+    uint32_t bad = p > hi ? 1u : 0u;
+    // the match of a sequence whose token nibble is mn and whose literals end at
+    // q, L words from output word k on; p = the next token
+    auto match = [&](uint32_t q, uint32_t mn, uint32_t k) {
+        const uint32_t y = lds32u(min(q, hi)), off = y & 0xFFFFu, rem = K - k;
+        uint32_t ml = mn + 4, q2 = q + 2, b = 0;
+        if (mn == 15) {
+            const uint32_t e = (y >> 16) & 255u, f = e == 255u ? y >> 24 : 0u;
+            ml += e + f;
+            q2 += e == 255u ? 2u : 1u;
+            b = f == 255u ? 1u : 0u;
+        }
+        M = ml >> 2;
+        b |= (q == block_end ? 1u : 0u) | (q2 > hi ? 1u : 0u) | ((off | ml) & 3u) | (off - 1u >= 4 * (k + L) ? 1u : 0u) |
+             (M > rem - L ? 1u : 0u);
+        bad |= L < rem ? b : 0u;  // (else the segment ends inside or right after the literals)
+        src = out + 4 * L - off;
+        p = q2;
+    };
+    if (info & 16u) {  // the segment starts inside a sequence
+        const uint32_t lit = info >> 5;
+        L = lit >> 2;
+        bad |= (lit & 3u) | (p + 4 * min(L, K) > hi ? 1u : 0u);
+        L = min(L, K);
+        if (active && !bad) match(p + 4 * L, info & 15u, 0);
+    }
+    bool run = active && !bad;
+    uint32_t k = 0;
+    while (__any_sync(0xFFFFFFFFu, run)) {
+        if (run && (L | M) == 0) {
+            const uint32_t x = lds32u(p), tok = x & 255u;
+            uint32_t lit = tok >> 4, q = p + 1;
+            bad = p >= hi ? 1u : 0u;
+            if (lit == 15) {
+                const uint32_t e = (x >> 8) & 255u, f = e == 255u ? (x >> 16) & 255u : 0u;
+                lit += e + f;
+                q += e == 255u ? 2u : 1u;
+                bad |= f == 255u ? 1u : 0u;
+            }
+            lp = q;
+            L = min(lit >> 2, K - k);
+            bad |= (lit & 3u) | (q + 4 * L > hi ? 1u : 0u);
+            match(q + lit, tok & 15u, k);
+            run = bad == 0;
+        }
+        if (run) {
+            // (a segment that ends inside a sequence's literals has M words it does not take)
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) {
+                const bool lt = L != 0;
+                if ((lt || M != 0) && k < K) {
+                    sts32(out, lds32u(lt ? lp : src));
+                    lp += lt ? 4u : 0u;
+                    src += lt ? 0u : 4u;
+                    L -= lt ? 1u : 0u;
+                    M -= lt ? 0u : 1u;
+                    out += 4;
+                    ++k;
+                }
+            }
+            run = k < K;
+        }
+    }
+    return !active || bad == 0;
 }
 
 // log2 of the lanes per segment for `nseg` segments on NT threads: the

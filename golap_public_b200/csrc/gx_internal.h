@@ -200,6 +200,7 @@ struct gx_column {
     uint32_t* d_bloom = nullptr;
     // LZ4: every block is one 16-byte aligned literal run (-1 = not known yet)
     mutable int lz4_direct = -1;
+    uint64_t lz4_seqs = 0;     // LZ4 with a fixed minimum match: sequences of the column, known when encoded
     bool casc_simple = false;  // cascaded: every page is simple (casc_page_simple), known when encoded
     int32_t* d_bmins = nullptr;
     int32_t* d_bmaxs = nullptr;

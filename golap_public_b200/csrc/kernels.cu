@@ -330,13 +330,15 @@ __device__ __forceinline__ int decode_tile(const gx_dcol& c, uint32_t slot, uint
             // pad words after each segment: G (groups of a warp on distinct
             // banks), 1 for a whole-warp group (its stores are contiguous)
             const uint32_t pl = glog == 5 ? 0u : glog;
-            const uint32_t gl = tid & (G - 1u), lane = tid & 31u;
-            const uint32_t gmask = G >= 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(G - 1u)));
-            for (uint32_t t = tid >> glog; t < nseg; t += (NT >> glog)) {
-                const uint32_t j = j0 + t;
+            const uint32_t gl = tid & (G - 1u);
+            // (whole warps go round together)
+            for (uint32_t t0 = (tid & ~31u) >> glog; t0 < nseg; t0 += (NT >> glog)) {
+                const uint32_t t = t0 + ((tid & 31u) >> glog);
+                const bool in = t < nseg;
+                const uint32_t j = j0 + (in ? t : 0u), ts = in ? t : 0u;
                 const uint32_t K = min(seg_rows, rows - j * seg_rows);
-                const int r2 = lz4_seg_group((const uint32_t*)stage, wbase, lo, hi, d.comp_bytes, seg_smem[2 * t],
-                                             seg_smem[2 * t + 1], K, buf + t * (seg_rows + (1u << pl)), gl, G, gmask);
+                const int r2 = lz4_seg_step((const uint32_t*)stage, wbase, lo, hi, d.comp_bytes, seg_smem[2 * ts],
+                                            seg_smem[2 * ts + 1], K, buf + ts * (seg_rows + (1u << pl)), gl, G, in);
                 if (r2 && gl == 0) *s_err = r2;
             }
             pad_log2 = pl;
@@ -2227,7 +2229,7 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     std::memset(&P, 0, sizeof(P));
     if (!shared_query(*plan, qd, cols, P.q, &why)) return GX_OK;
     if (cols.size() > kWsMaxCols) return GX_OK;
-    uint32_t areas = 0;
+    uint32_t areas = 0, other = 0;  // words of decode buffers per warp; columns decoded one by one
     bool cut_tiles = true;  // parts of a tile would each decode the whole tile's LZ4 segments
     for (size_t i = 0; i < kWsMaxCols; ++i) P.buf_of[i] = kWsNone;
     for (size_t i = 0; i < cols.size(); ++i) {
@@ -2245,9 +2247,26 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
         }
         if (!(c->codec == GX_CODEC_NONE || (c->codec == GX_CODEC_LZ4 && lz4_all_direct(c)) ||
               (c->codec == GX_CODEC_CASCADED && c->casc_simple))) {
-            P.buf_of[i] = areas++;
             if (c->codec == GX_CODEC_LZ4) cut_tiles = false;
+            // a lane per segment: at least three sequences to eight rows (1.5 words a sequence, Q1
+            // over 10M rows: 320 us, 570 with lz4_seg_step; 4 words, 6M rows: 250 and 168)
+            if (c->codec == GX_CODEC_LZ4 && c->seg_shift >= kWsLaneShift0 && c->seg_shift <= kWsLaneShift1 &&
+                c->lz4_seqs * 8 >= c->n_rows * 3) {
+                P.lane_cols |= 1u << i;
+                P.buf_of[i] = areas;
+                areas += kWsTile + (kWsTile >> c->seg_shift) * 4;
+            } else {
+                other |= 1u << i;
+            }
         }
+    }
+    // the other columns' buffers; the first lies where the lane columns' ranges
+    // are staged, which they have left when it is written
+    P.stage_of = areas;
+    uint32_t behind = 0;  // words after the staging area
+    for (uint32_t m = other; m; m &= m - 1) {
+        P.buf_of[__builtin_ctz(m)] = areas + behind;  // (moved behind the stages below, but for the first)
+        behind += kWsTile;
     }
     P.q.keep_in = plan->keep_chunks_dev;
     P.q.keep_out = plan->keep_out_dev;
@@ -2268,8 +2287,28 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     if (P.chunk_words > kWsMaxChunkWords) return GX_OK;
     // the kernel indexes tiles in 32 bits (with room for its stride)
     if ((uint64_t)n_range * P.blocks_per_chunk * P.tiles_per_block >= (1ull << 31)) return GX_OK;
-    P.n_areas = areas;
     P.grouped_tab = P.q.grouped ? 1u : 0u;
+    // staging buffers of the LZ4 columns that take a lane per segment (up to four
+    // columns share the lanes): the most CTAs per SM for the passes a tile takes
+    const uint32_t first_buf = other ? kWsTile : 0u;
+    auto warp_words = [&](uint32_t stages) {
+        return kWsHead + (P.grouped_tab ? kWsQueueWords : 0u) + areas + std::max(stages * kWsStageWords, first_buf) +
+               behind - first_buf;
+    };
+    auto smem_of = [&](uint32_t stages) {
+        return 4ull * (2ull * P.chunk_words + (size_t)warp_words(stages) * kWsWarps +
+                       (P.grouped_tab ? 3ull * kWsGroupSlots : 0ull));
+    };
+    if (P.lane_cols) {
+        const size_t sm = 225u << 10, fixed = 2u << 10;  // per SM, and static and reserved per CTA
+        P.n_stages = 1;
+        const uint32_t n_lane = (uint32_t)__builtin_popcount(P.lane_cols);
+        auto rate = [&](uint32_t k) { return 12 * (sm / (smem_of(k) + fixed)) / ((n_lane + k - 1) / k); };
+        for (uint32_t k = 2; k <= 4 && k <= n_lane; ++k)
+            if (rate(k) >= rate(P.n_stages)) P.n_stages = k;
+        const uint32_t room = std::max(P.n_stages * kWsStageWords, first_buf) - first_buf;
+        for (uint32_t m = other & (other - 1); m; m &= m - 1) P.buf_of[__builtin_ctz(m)] += room;
+    }
     P.rows_scanned = rows_dev;
     // the plan's signature: a compile-time evaluator when one matches
     uint32_t kinds[GX_MAX_STEPS] = {};
@@ -2287,9 +2326,8 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     else if (sig == kSigQ3) kern = warp_scan_kernel<kSigQ3>;
     else if (sig == kSigQ4) kern = warp_scan_kernel<kSigQ4>;
     else if (sig == kSigGroup) kern = warp_scan_kernel<kSigGroup>;
-    P.warp_words = kWsHead + (P.grouped_tab ? kWsQueueWords : 0u) + areas * kWsTile;
-    const size_t smem = 4ull * (2ull * P.chunk_words + (size_t)P.warp_words * kWsWarps +
-                                (P.grouped_tab ? 3ull * kWsGroupSlots : 0ull));
+    P.warp_words = warp_words(P.n_stages);
+    const size_t smem = smem_of(P.n_stages);
     if (smem > kWsMaxDynSmem) return GX_OK;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWsNT, smem) != cudaSuccess || per_sm < 1)

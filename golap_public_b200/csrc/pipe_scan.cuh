@@ -245,13 +245,14 @@ __device__ __forceinline__ int pipe_lz4_tile(const gx_dcol& c, const PipeTile& T
     while (glog > 0 && glog < 5 && (nseg << glog) > 256u) --glog;
     const uint32_t G = 1u << glog;
     const uint32_t pl = glog == 5 ? 0u : glog;
-    const uint32_t gl = tid & (G - 1u), lane = tid & 31u;
-    const uint32_t gmask = G >= 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(G - 1u)));
-    for (uint32_t t = tid >> glog; t < nseg; t += (kPipeNC >> glog)) {
-        const uint32_t j = j0 + t;
+    const uint32_t gl = tid & (G - 1u);
+    for (uint32_t t0 = (tid & ~31u) >> glog; t0 < nseg; t0 += (kPipeNC >> glog)) {  // whole warps go round together
+        const uint32_t t = t0 + ((tid & 31u) >> glog);
+        const bool in = t < nseg;
+        const uint32_t ts = in ? t : 0u, j = j0 + ts;
         const uint32_t K = min(seg_rows, T.rows - j * seg_rows);
-        const int r2 = lz4_seg_group((const uint32_t*)area, wbase, pc.lo, pc.hi, pc.end, s_seg[2 * t],
-                                     s_seg[2 * t + 1], K, buf + t * (seg_rows + (1u << pl)), gl, G, gmask);
+        const int r2 = lz4_seg_step((const uint32_t*)area, wbase, pc.lo, pc.hi, pc.end, s_seg[2 * ts],
+                                    s_seg[2 * ts + 1], K, buf + ts * (seg_rows + (1u << pl)), gl, G, in);
         if (r2 && gl == 0) *s_err = r2;
     }
     return (int)pl;

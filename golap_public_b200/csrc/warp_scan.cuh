@@ -74,6 +74,13 @@ constexpr uint32_t kWsMaxChunkWords = 1024;     // chunk keep bits of one launch
 // step (16), the constant steps' group-key digits (32), the rows scanned (2,
 // and 2 of padding)
 constexpr uint32_t kWsHead = 32 * 8 + 8 * 8 + 2 * GX_MAX_STEPS + 32 + 4;
+// LZ4 columns decoded with one lane per segment: segments of 32 to 128 rows,
+// four words of padding after each; the staged compressed bytes of a tile
+// (less than 7/8 of its rows' bytes, and the ends of the aligned copy)
+constexpr uint32_t kWsLaneShift0 = 5, kWsLaneShift1 = 7;
+constexpr uint32_t kWsLaneWords = kWsTile + (kWsTile >> kWsLaneShift0) * 4;
+constexpr uint32_t kWsStageWords = kWsTile * 7 / 8 + 16;
+static_assert(4 * kWsStageWords >= 4 * kWsTile * 7 / 8 + 38 && kWsStageWords % 4 == 0, "a staged range fits");
 constexpr uint32_t kWsQueueWords = (kWsBatch + 32) * 3;  // grouped plans: the warp's WsQueue, before its decode buffers
 static_assert(kWsHead % 4 == 0, "decode buffers start 16-byte aligned");
 static_assert(kWsTile == kCascTileRows, "simple cascaded pages are simple for the scan's tiles");
@@ -90,8 +97,10 @@ struct WsParams {
     uint32_t parts;                 // 1: tiles of the last round may be cut (no column needs an LZ4 decode)
     uint64_t n_rows;                // rows of the table
     uint32_t chunk_lo, chunk_hi;    // chunks [chunk_lo, chunk_hi) are scanned
-    uint32_t buf_of[kWsMaxCols];    // decode buffer of column c (cascaded / LZ4 with matches), or kWsNone
-    uint32_t n_areas;               // decode buffers per warp (kWsTile words each)
+    uint32_t buf_of[kWsMaxCols];    // decode buffer of column c (cascaded / LZ4 with matches): word in the warp's
+                                    // areas, or kWsNone
+    uint32_t lane_cols;             // LZ4 columns of short sequences (a lane per segment)
+    uint32_t stage_of, n_stages;    // staging of their compressed ranges: first word, buffers of kWsStageWords
     uint32_t warp_words;            // shared memory words per warp
     uint32_t chunk_words;           // words of the chunk keep bitmap (and of its prefix counts)
     uint32_t grouped_tab;           // 1: the warp has a group table
@@ -221,20 +230,115 @@ __device__ __noinline__ int ws_lz4_rows(const uint8_t* blk, uint32_t blk_bytes, 
     const uint32_t glog = seg_group_log2(nseg, 32);
     const uint32_t G = 1u << glog;
     const uint32_t gl = lane & (G - 1u);
-    const uint32_t gmask = G >= 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(G - 1u)));
+    // the tile's compressed lines into L1 first, all in flight together
+    for (uint32_t x = 128 * lane; x < hi - lo; x += 128 * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(A + x / 4));
     int err = 0;
     for (uint32_t t0 = 0; t0 < nseg; t0 += (32u >> glog)) {
         const uint32_t t = t0 + (lane >> glog);
-        if (t < nseg) {
-            const uint32_t j = j0 + t;
-            const uint32_t K = min(seg_rows, rows - j * seg_rows);
-            const uint32_t cp = __ldg(e + 2 * j), info = __ldg(e + 2 * j + 1);
-            const int r = lz4_seg_group(A, wbase, lo, hi, blk_bytes, cp, info, K, out + t * seg_rows, gl, G, gmask);
-            if (r) err = r;
-        }
+        const bool in = t < nseg;
+        const uint32_t j = j0 + (in ? t : 0u);
+        const uint32_t K = min(seg_rows, rows - j * seg_rows);
+        const uint32_t cp = __ldg(e + 2 * j), info = __ldg(e + 2 * j + 1);
+        if (lz4_seg_step(A, wbase, lo, hi, blk_bytes, cp, info, K, out + (in ? t : 0u) * seg_rows, gl, G, in))
+            err = kErrCorrupt;
     }
     __syncwarp();
     return __any_sync(0xFFFFFFFFu, err != 0) ? kErrCorrupt : 0;
+}
+
+// One row tile: block slot, first row in the block, rows, block rows, and
+// the rows [a, b) of the tile that the warp evaluates (all of them, or the
+// part of a tile cut for the last round).
+struct __align__(16) WsTile {
+    uint32_t slot, r0, n, rows, a, b;
+    uint32_t steps;  // bit s: step s is over a constant column; kWsDead, kWsBroadcast
+    uint32_t pad;
+};
+constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
+constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a loose step's that is not packed
+static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
+
+// How one column of one tile is read.
+struct __align__(16) WsCol {
+    const uint8_t* src;   // direct, kWmRows: the rows; LZ4: the block; cascaded: the page; kWmPack: its values
+    uint32_t mode;        // kWm*
+    int32_t cval;         // kWmConst: the value; kWmRuns2: the first run's; kWmPack: the frame of reference
+    uint32_t aux0, aux1;  // LZ4: [lo, hi) in the block; cascaded: page bytes, page rows; kWmRuns2: the first
+                          // run's end, the second's value; kWmPack: bits per value; kWmRows: log2 of the rows
+                          // between every four words of padding
+    uint32_t bytes;       // LZ4: the block's compressed bytes; kWmPack: the tile's first row in the page
+    uint32_t pad;
+};
+static_assert(sizeof(WsCol) == 32, "column records of 8 words");
+
+// Four rows of a column read in place (16-byte aligned), without taking room
+// in L1.  (volatile: the loads of a batch stay together at
+// its start, also when a value is used only after the probes.)
+__device__ __forceinline__ uint4 ws_ld_rows(const uint8_t* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+
+// The tile's LZ4 columns of short sequences (P.lane_cols; unless nearly all
+// literals on this tile) decoded with one lane per segment: up to n_stages
+// columns at a time, as many as have 32 segments on the tile together.  Their
+// compressed ranges are staged, their rows land with four words between
+// segments (cols[c].aux0 = log2 of the segment).  Returns the columns done;
+// *err is set on a corrupt stream.
+__device__ __noinline__ uint32_t ws_lz4_lanes(const WsParams& P, const gx_dcol* s_cols, const WsTile& T, WsCol* cols,
+                                              uint32_t todo, uint32_t* areas, uint32_t lane, int* err) {
+    uint32_t done = 0;
+    // the columns that qualify: lane c decides column c
+    bool q = false;
+    if ((todo >> lane) & 1u) {
+        q = (cols[lane].aux1 - cols[lane].aux0) * 8 < T.n * 4 * 7;
+    }
+    todo = __ballot_sync(0xFFFFFFFFu, q);
+    while (todo) {
+        // one pass: columns of one segment size
+        const uint32_t shift = s_cols[__ffs(todo) - 1].seg_shift, nseg = (T.n + (1u << shift) - 1) >> shift;
+        uint32_t pass = 0, cnt = 0, mine = kWsNone, my_stage = 0;
+        for (uint32_t m = todo; m && cnt < P.n_stages && (cnt + 1) * nseg <= 32; m &= m - 1) {
+            const uint32_t c = __ffs(m) - 1;
+            if (s_cols[c].seg_shift != shift) continue;
+            uint32_t* st = areas + P.stage_of + cnt * kWsStageWords;
+            const uintptr_t a0 = ((uintptr_t)cols[c].src + cols[c].aux0) & ~(uintptr_t)15;
+            const uintptr_t a1 = (uintptr_t)cols[c].src + cols[c].aux1;
+            // (up to 23 bytes past the range: inside the payload's slack)
+            for (uint32_t i = lane; i < (uint32_t)(a1 - a0 + 8 + 15) / 16; i += 32)
+                ((uint4*)st)[i] = ws_ld_rows((const uint8_t*)a0 + 16 * i);
+            if (lane / nseg == cnt) {
+                mine = c;
+                my_stage = smem_u32(st) + (uint32_t)((uintptr_t)cols[c].src + cols[c].aux0 - a0) - cols[c].aux0;
+            }
+            pass |= 1u << c;
+            ++cnt;
+        }
+        const bool in = mine != kWsNone && lane < cnt * nseg;
+        const uint32_t c = in ? mine : (uint32_t)__ffs(pass) - 1, t = in ? lane % nseg : 0u;
+        const gx_dcol& col = s_cols[c];
+        const uint32_t j = (T.r0 >> shift) + t, K = min(1u << shift, T.rows - (j << shift));
+        const uint32_t* e = col.seg + (size_t)2 * col.S * T.slot + 2 * j;
+        const uint32_t cp = __ldg(e), info = __ldg(e + 1), lo = cols[c].aux0, hi = cols[c].aux1;
+        const bool range = cp >= lo && cp <= hi;
+        __syncwarp();
+        const bool ok = lz4_seg_lane(my_stage + (range ? cp : lo), my_stage + hi, my_stage + cols[c].bytes, info, K,
+                                     smem_u32(areas + P.buf_of[c] + t * ((1u << shift) + 4)), in && range);
+        if (__any_sync(0xFFFFFFFFu, in && !(ok && range))) *err = kErrCorrupt;
+        __syncwarp();
+        if (lane < 8 && ((pass >> lane) & 1u)) {
+            cols[lane].mode = kWmRows;
+            cols[lane].src = (const uint8_t*)(areas + P.buf_of[lane]);
+            cols[lane].aux0 = shift;
+        }
+        __syncwarp();
+        done |= pass;
+        todo &= ~pass;
+    }
+    return done;
 }
 
 // Add of (key, val) to the CTA's group table in shared memory: sets of four
@@ -320,30 +424,6 @@ __device__ __forceinline__ uint32_t ws_select(uint32_t m, uint32_t k) {
     }
     return pos;
 }
-
-// One row tile: block slot, first row in the block, rows, block rows, and
-// the rows [a, b) of the tile that the warp evaluates (all of them, or the
-// part of a tile cut for the last round).
-struct __align__(16) WsTile {
-    uint32_t slot, r0, n, rows, a, b;
-    uint32_t steps;  // bit s: step s is over a constant column; kWsDead, kWsBroadcast
-    uint32_t pad;
-};
-constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
-constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a loose step's that is not packed
-static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
-
-// How one column of one tile is read.
-struct __align__(16) WsCol {
-    const uint8_t* src;   // direct, kWmRows: the rows; LZ4: the block; cascaded: the page; kWmPack: its values
-    uint32_t mode;        // kWm*
-    int32_t cval;         // kWmConst: the value; kWmRuns2: the first run's; kWmPack: the frame of reference
-    uint32_t aux0, aux1;  // LZ4: [lo, hi) in the block; cascaded: page bytes, page rows; kWmRuns2: the first
-                          // run's end, the second's value; kWmPack: bits per value
-    uint32_t bytes;       // LZ4: the block's compressed bytes; kWmPack: the tile's first row in the page
-    uint32_t pad;
-};
-static_assert(sizeof(WsCol) == 32, "column records of 8 words");
 
 // n / d for n < 2^31, d's multiplier and shift computed by the host.
 __device__ __forceinline__ uint32_t ws_div(uint32_t n, uint32_t mul, uint32_t shift) {
@@ -710,17 +790,6 @@ constexpr uint32_t ws_probes_end(uint32_t sig) {
 template <uint32_t SIG>
 constexpr uint32_t kWsProbesEnd = ws_probes_end(SIG);
 
-// Four rows of a column read in place (16-byte aligned), without taking room
-// in L1.  (volatile: the loads of a batch stay together at
-// its start, also when a value is used only after the probes.)
-__device__ __forceinline__ uint4 ws_ld_rows(const uint8_t* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
-}
-
 // Elements i .. i + 3 of a bit-packed stream of width w (1..32), plus base:
 // the words that hold them are shifted to the first one's bit once (s below,
 // per lane), after which element k starts at bit k * w in every lane.  Reads
@@ -759,6 +828,11 @@ __device__ __forceinline__ uint4 ws_runs2(const WsCol& d, uint32_t row) {
     return make_uint4(row < e ? v0 : v1, row + 1 < e ? v0 : v1, row + 2 < e ? v0 : v1, row + 3 < e ? v0 : v1);
 }
 
+// Tile rows row .. row + 3 of a decoded column.
+__device__ __forceinline__ uint4 ws_decoded(const WsCol& d, uint32_t row) {
+    return *(const uint4*)(d.src + 4 * (row + ((row >> d.aux0) << 2)));
+}
+
 // Tile rows row .. row + 3 of a column, however it is read.
 __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
     const uint32_t mode = d.mode;
@@ -767,7 +841,7 @@ __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
     const uint32_t v0 = (uint32_t)d.cval;
     if (mode == kWmConst) return make_uint4(v0, v0, v0, v0);
     if (mode == kWmRuns2) return ws_runs2(d, row);
-    return *(const uint4*)(d.src + 4 * row);  // kWmRows
+    return ws_decoded(d, row);  // kWmRows
 }
 
 // Tile rows [a, b) evaluated through the plan's steps, H 128-row groups at a
@@ -837,7 +911,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
                         if (loose && !skip && d.mode == kWmRuns2)
                             x = ws_runs2(d, row + kWsBatch * h);
                         else if (loose && !skip && d.mode == kWmRows)
-                            x = *(const uint4*)(d.src + 4 * (row + kWsBatch * h));
+                            x = ws_decoded(d, row + kWsBatch * h);
                         else if (!skip)
                             x = ws_ld_rows(src[s] + kWsBatch * 4 * h);
                     } else if (cols[Q.steps[s].col].mode == kWmDirect && row + kWsBatch * h < b) {
@@ -1039,7 +1113,7 @@ __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __
     uint32_t* const wdig = wmem + 40 * 8 + 2 * GX_MAX_STEPS;  // constant steps' group-key digits
     unsigned long long* const wrows = (unsigned long long*)(wdig + 32);  // rows scanned
     WsQueue* const wq = (WsQueue*)(wmem + kWsHead);          // grouped: rows on their way to the group table
-    uint32_t* const areas = wmem + kWsHead + (P.grouped_tab ? kWsQueueWords : 0u);  // n_areas x kWsTile words
+    uint32_t* const areas = wmem + kWsHead + (P.grouped_tab ? kWsQueueWords : 0u);  // the decode buffers
     // grouped: the CTA's group table (keys, low halves, high halves of the sums) after the warps' regions
     uint32_t* const tkey = s_kpre + P.chunk_words + (size_t)kWsWarps * P.warp_words;
     const uint64_t pol_keep = ws_policy_keep();
@@ -1146,16 +1220,19 @@ __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __
             if (!((vm >> q) & 1u)) continue;
             const WsTile& T = wtiles[q];
             WsCol* const cols = wcols + (q << cl);
-            // ---- decodes, one column at a time by the whole warp
+            // ---- decodes: LZ4 columns of short sequences together, the others one
+            // at a time by the whole warp
             int terr = 0;
-            for (uint32_t c = 0; c < ncols; ++c) {
+            const uint32_t lz = __ballot_sync(0xFFFFFFFFu, lane < ncols && cols[lane].mode == kWmLz4);
+            if (lz & P.lane_cols) ws_lz4_lanes(P, s_cols, T, cols, lz & P.lane_cols, areas, lane, &terr);
+            for (uint32_t c = 0; c < ncols && !terr; ++c) {
                 const uint32_t m = cols[c].mode;
                 if (m == kWmBad) {
                     terr = kErrCorrupt;
                     break;
                 }
                 if (m != kWmLz4 && m != kWmCasc) continue;
-                uint32_t* buf = areas + (size_t)P.buf_of[c] * kWsTile;
+                uint32_t* buf = areas + P.buf_of[c];
                 int32_t cv = 0;
                 int r = 0;
                 if (m == kWmCasc) {
@@ -1178,6 +1255,7 @@ __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __
                 if (lane == 0) {
                     cols[c].mode = kWmRows;
                     cols[c].src = (const uint8_t*)buf;
+                    cols[c].aux0 = 31;  // no padding
                 }
                 __syncwarp();
             }

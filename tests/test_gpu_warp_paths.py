@@ -119,3 +119,54 @@ def test_group_by_of_a_range(cuda, n, date):
             api.scan_check()
     else:
         api.scan_check()
+
+
+@pytest.mark.parametrize("rpb,S", [(4096, 128), (8192, 128), (16384, 128), (16384, 32)])
+@pytest.mark.parametrize("n", [31, 1025, 70_003])
+def test_short_sequences(cuda, rpb, S, n):
+    # LZ4 segments of 32, 64, 128 and 512 rows full of short matches: one to
+    # three such columns beside a literal one, with literal runs longer than one
+    # and two extension bytes, and matches longer than a token's nibble
+    r = np.random.default_rng(n + S)
+    kw = dict(rows_per_block=rpb, lz4_segments=S, lz4_min_match=4)
+    few = r.integers(0, 5, n)
+    mixed = np.where(r.integers(0, 400, n) < 3, r.integers(-2**31, 2**31, n), r.integers(0, 9, n))
+    bursts = r.integers(0, 2**31, n)
+    bursts[(np.arange(n) // 40) % 3 != 0] = 7
+    cols = [_col(x, "lz4", **kw) for x in (few, mixed, bursts)]
+    price = r.integers(0, 2**31, n)
+    cp = _col(price, "lz4", rows_per_block=rpb, lz4_segments=S)
+    m = (few >= 1) & (few <= 3)
+    assert _sum(cuda, cols[0], 1, 3, cp) == int(price[m].sum())
+    assert _sum(cuda, cols[0], 1, 3, cols[1]) == int(mixed[m].sum())
+    m &= (mixed >= 2) & (mixed <= 6)
+    res = cuda.zeros(1, dtype=cuda.int64, device="cuda")
+    p = api.ScanPlan(agg=L.GX_AGG_SUM_PRODUCT, result=res)
+    p.filter(cols[0], 1, 3, carry=True).filter(cols[1], 2, 6).value(cols[2])
+    p.launch()
+    api.scan_check()
+    assert int(res.item()) == int((few[m] * bursts[m]).sum())
+
+
+@pytest.mark.parametrize("n", [2_000, 70_000])
+def test_short_sequences_corrupt(cuda, n):
+    # flipped bytes either decode to other values or are reported, and the
+    # library works afterwards
+    r = np.random.default_rng(n)
+    v, x = r.integers(0, 11, n), r.integers(0, 100, n)
+    cx = _col(x, "none")
+    reported = 0
+    for trial in range(16):
+        col = api.Column(v.astype(np.int32), "lz4", rows_per_chunk=40_000, lz4_min_match=4)
+        pay = col.payload_view()
+        b = col.blocks()[trial % col.info.n_blocks]
+        at = int(b[0]) + int(r.integers(0, int(b[2])))
+        pay[at] = 255 if trial % 2 else int(r.integers(0, 256))
+        col.to_device()
+        try:
+            _sum(cuda, col, 2, 8, cx)
+        except api.L.GxError as e:
+            assert e.status == L.GX_ERR_CORRUPT
+            reported += 1
+    assert reported >= 1
+    assert _sum(cuda, _col(v, "lz4", lz4_min_match=4), 2, 8, cx) == int(x[(v >= 2) & (v <= 8)].sum())

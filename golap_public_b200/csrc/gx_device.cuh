@@ -683,6 +683,63 @@ __device__ __forceinline__ bool ht_probe_any(const uint64_t* __restrict__ slots,
     return layout ? ht_probe_bucket(slots, log2cap, key, payload) : ht_probe(slots, log2cap, key, payload);
 }
 
+// A join-table probe of R rows per lane (hdr: a dense table's header): rows whose bit
+// in m is set and whose key is found keep their bit, with their payload in
+// pay.  All rows' reads of a round are in flight together, a round reads two
+// neighbouring slots (16 bytes, one sector) and goes on with the rows whose
+// chain is not settled.  The three layouts are one walk: linear tables from
+// the key's hash slot, bucket tables from the first slot of its bucket (keys
+// fill a bucket's slots in order, then the next bucket's), dense tables one
+// slot.  A pair's slot before the key's own can hold the key only in a dense
+// table's header (its base), so the slot at or after it is preferred.
+template <uint32_t R>
+__device__ __forceinline__ uint32_t ht_probe_rows(const uint64_t* __restrict__ ht, uint32_t log2cap, uint32_t lay,
+                                                  uint64_t hdr, const uint32_t (&v)[R], uint32_t m,
+                                                  uint32_t (&pay)[R], uint64_t pol) {
+    const uint32_t mask = (1u << log2cap) - 1u;
+    const bool dense = lay == GX_HT_DENSE;
+    uint32_t slot[R];
+#pragma unroll
+    for (uint32_t r = 0; r < R; ++r) {
+        bool out = v[r] == (uint32_t)kEmptyKey;
+        if (dense) {
+            const uint32_t u = v[r] - (uint32_t)hdr;
+            out = out || u >= (uint32_t)(hdr >> 32);
+            slot[r] = 1u + u;
+        } else if (lay == GX_HT_BUCKET) {
+            slot[r] = hash_key32((int32_t)v[r], log2cap - 3) * kBucketSlots;
+        } else {
+            slot[r] = hash_key32((int32_t)v[r], log2cap);
+        }
+        if (out) m &= ~(1u << r);
+    }
+    uint32_t u = m;  // rows whose chain is not settled
+#pragma unroll 1
+    for (uint32_t t = 0; u && t <= mask / 2 + 1; ++t) {
+        ulonglong2 e[R];
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) {
+            asm("" : "=l"(e[r].x), "=l"(e[r].y));  // rows not read keep any value: masked below
+            if ((u >> r) & 1u)
+                asm("ld.global.nc.L2::cache_hint.v2.b64 {%0, %1}, [%2], %3;"
+                    : "=l"(e[r].x), "=l"(e[r].y)
+                    : "l"(ht + (slot[r] & ~1u)), "l"(pol));
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) {
+            const uint32_t bit = 1u << r, kx = (uint32_t)e[r].x, ky = (uint32_t)e[r].y;
+            const bool hit = kx == v[r] || ky == v[r];
+            const bool open = !hit && !dense && ky != (uint32_t)kEmptyKey &&
+                              (kx != (uint32_t)kEmptyKey || (slot[r] & 1u));
+            if ((u & bit) && hit) pay[r] = ky == v[r] ? (uint32_t)(e[r].y >> 32) : (uint32_t)(e[r].x >> 32);
+            if ((u & bit) && !hit && !open) m &= ~bit;
+            if (!open) u &= ~bit;
+            slot[r] = ((slot[r] | 1u) + 1u) & mask;
+        }
+    }
+    return m & ~u;
+}
+
 // --------------------------------------------------------- group tables
 // Global open-addressing group table: keys int64 (kEmptyGroup = free), sums int64.
 __device__ __forceinline__ bool group_add_global(int64_t* keys, int64_t* sums, uint32_t log2cap, int64_t key,

@@ -251,9 +251,10 @@ __device__ __noinline__ int ws_lz4_rows(const uint8_t* blk, uint32_t blk_bytes, 
 // part of a tile cut for the last round).
 struct __align__(16) WsTile {
     uint32_t slot, r0, n, rows, a, b;
-    uint32_t steps;  // bit s: step s is over a constant column; kWsDead, kWsBroadcast
+    uint32_t steps;  // bit s: step s is over a constant column; kWsDecode, kWsDead, kWsMixed
     uint32_t pad;
 };
+constexpr uint32_t kWsDecode = 1u << 29;     // a column needs a decode, or is corrupt
 constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
 constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a loose step's that is not packed
 static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
@@ -339,6 +340,44 @@ __device__ __noinline__ uint32_t ws_lz4_lanes(const WsParams& P, const gx_dcol* 
         todo &= ~pass;
     }
     return done;
+}
+
+// The columns of a tile that need a decode (or are corrupt), by the whole warp:
+// LZ4 columns of short sequences together, the others one at a time.  Returns
+// 0 or the error.  Out of line: most tiles have none.
+__device__ __noinline__ int ws_decode_tile(const WsParams& P, const gx_dcol* s_cols, const WsTile& T, WsCol* cols,
+                                           uint32_t* areas, uint32_t lane) {
+    const uint32_t ncols = P.n_cols;
+    int terr = 0;
+    const uint32_t lz = __ballot_sync(0xFFFFFFFFu, lane < ncols && cols[lane].mode == kWmLz4);
+    if (lz & P.lane_cols) ws_lz4_lanes(P, s_cols, T, cols, lz & P.lane_cols, areas, lane, &terr);
+    for (uint32_t c = 0; c < ncols && !terr; ++c) {
+        const uint32_t m = cols[c].mode;
+        if (m == kWmBad) return kErrCorrupt;
+        if (m != kWmLz4 && m != kWmCasc) continue;
+        uint32_t* buf = areas + P.buf_of[c];
+        int32_t cv = 0;
+        if (m == kWmCasc) {
+            terr = ws_casc_rows(cols[c].src, cols[c].aux0, cols[c].aux1, T.r0 & (kCascPageRows - 1u), T.n,
+                                (int32_t*)buf, &cv, lane);
+            if (terr == 1) {  // one run covers the tile (a page of many runs): its value written out
+                for (uint32_t i = lane; i < T.n; i += 32) buf[i] = (uint32_t)cv;
+                terr = 0;
+            }
+        } else {
+            const gx_dcol& col = s_cols[c];
+            terr = ws_lz4_rows(cols[c].src, cols[c].bytes, col.seg + (size_t)2 * col.S * T.slot, col.seg_shift, T.rows,
+                               T.r0, T.n, cols[c].aux0, cols[c].aux1, buf, lane);
+        }
+        __syncwarp();
+        if (lane == 0) {
+            cols[c].mode = kWmRows;
+            cols[c].src = (const uint8_t*)buf;
+            cols[c].aux0 = 31;  // no padding
+        }
+        __syncwarp();
+    }
+    return terr;
 }
 
 // Add of (key, val) to the CTA's group table in shared memory: sets of four
@@ -663,7 +702,11 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
                                                uint32_t lane) {
     const ShQuery& Q = P.q;
     const uint32_t cl = P.col_log2, q = lane >> cl, s = lane & ((1u << cl) - 1u);
-    bool isc = false, ok = true, bad = false, mixed = false;
+    bool isc = false, ok = true, bad = false, mixed = false, dec = false;
+    if (((vm >> q) & 1u) && s < P.n_cols) {  // as a column
+        const uint32_t m = cols[lane].mode;
+        dec = m == kWmLz4 || m == kWmCasc || m == kWmBad;
+    }
     if (((vm >> q) & 1u) && s < Q.n_steps) {
         const ShStep& st = Q.steps[s];
         const WsCol& c = cols[(q << cl) + st.col];
@@ -687,9 +730,10 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
     const uint32_t cst = (__ballot_sync(0xFFFFFFFFu, isc) >> sh) & m0;
     const uint32_t fails = (__ballot_sync(0xFFFFFFFFu, isc && !ok) >> sh) & m0;
     const uint32_t bads = (__ballot_sync(0xFFFFFFFFu, bad) >> sh) & m0;
+    const uint32_t decs = (__ballot_sync(0xFFFFFFFFu, dec) >> sh) & m0;
     const uint32_t mixes = (__ballot_sync(0xFFFFFFFFu, mixed) >> sh) & m0;
     if (s == 0 && ((vm >> q) & 1u)) {
-        uint32_t f = cst | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
+        uint32_t f = cst | (decs ? kWsDecode : 0u) | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
         if (SIG != 0 && bads) {
             // a digit out of range is an error unless a constant step before it drops
             // the rows; the run-time evaluator raises it only for rows alive at the step
@@ -1163,45 +1207,8 @@ __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __
             if (!((vm >> q) & 1u)) continue;
             const WsTile& T = wtiles[q];
             WsCol* const cols = wcols + (q << cl);
-            // ---- decodes: LZ4 columns of short sequences together, the others one
-            // at a time by the whole warp
             int terr = 0;
-            const uint32_t lz = __ballot_sync(0xFFFFFFFFu, lane < ncols && cols[lane].mode == kWmLz4);
-            if (lz & P.lane_cols) ws_lz4_lanes(P, s_cols, T, cols, lz & P.lane_cols, areas, lane, &terr);
-            for (uint32_t c = 0; c < ncols && !terr; ++c) {
-                const uint32_t m = cols[c].mode;
-                if (m == kWmBad) {
-                    terr = kErrCorrupt;
-                    break;
-                }
-                if (m != kWmLz4 && m != kWmCasc) continue;
-                uint32_t* buf = areas + P.buf_of[c];
-                int32_t cv = 0;
-                int r = 0;
-                if (m == kWmCasc) {
-                    r = ws_casc_rows(cols[c].src, cols[c].aux0, cols[c].aux1, T.r0 & (kCascPageRows - 1u), T.n,
-                                     (int32_t*)buf, &cv, lane);
-                    if (r == 1) {  // one run covers the tile (a page of many runs): its value written out
-                        for (uint32_t i = lane; i < T.n; i += 32) buf[i] = (uint32_t)cv;
-                        r = 0;
-                    }
-                } else {
-                    const gx_dcol& col = s_cols[c];
-                    r = ws_lz4_rows(cols[c].src, cols[c].bytes, col.seg + (size_t)2 * col.S * T.slot, col.seg_shift,
-                                    T.rows, T.r0, T.n, cols[c].aux0, cols[c].aux1, buf, lane);
-                }
-                __syncwarp();
-                if (r) {
-                    terr = r;
-                    break;
-                }
-                if (lane == 0) {
-                    cols[c].mode = kWmRows;
-                    cols[c].src = (const uint8_t*)buf;
-                    cols[c].aux0 = 31;  // no padding
-                }
-                __syncwarp();
-            }
+            if (T.steps & kWsDecode) terr = ws_decode_tile(P, s_cols, T, cols, areas, lane);
             if (terr) {
                 if (lane == 0) raise_error(terr);
                 continue;

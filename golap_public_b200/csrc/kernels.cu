@@ -951,21 +951,30 @@ __global__ void ht_build_kernel(uint64_t* slots, uint32_t log2cap, const int32_t
     ht_count(ins, dup, bad, counters);
 }
 
-// A small linear table in one launch: one CTA clears the slots and the
-// counters, then inserts (dimension tables such as the date table).
+// A small linear table in one launch of one CTA (dimension tables such as the
+// date table).  Up to kSmemHtSlots slots it is built in shared memory and
+// written out whole: the chains of compare-and-swaps then take shared-memory
+// latency (2,556 dates into 8,192 slots: 9.0 us in global memory, 7.0 us; 31 of
+// them 4.6 us); larger ones are cleared and filled in place.
 constexpr uint64_t kSmallHtSlots = 1u << 16, kSmallHtRows = 1u << 16;
-__global__ void ht_build_small_kernel(uint64_t* slots, uint32_t log2cap, const int32_t* keys, const int32_t* payload,
-                                      uint64_t n, const __grid_constant__ BuildPreds preds,
-                                      unsigned long long* counters) {
+constexpr uint32_t kSmemHtSlots = 1u << 13;
+template <bool SMEM>
+__global__ void __launch_bounds__(1024) ht_build_small_kernel(uint64_t* slots, uint32_t log2cap, const int32_t* keys,
+                                                              const int32_t* payload, uint64_t n,
+                                                              const __grid_constant__ BuildPreds preds,
+                                                              unsigned long long* counters) {
+    extern __shared__ __align__(16) uint64_t s_slots[];
     griddep_launch();  // a scan launched after the build may start its table-free work now
-    const uint64_t cap = 1ull << log2cap;  // at least 16
-    for (uint64_t i = threadIdx.x; i < cap / 2; i += blockDim.x)
-        ((ulonglong2*)slots)[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
+    const uint32_t cap = 1u << log2cap;  // at least 16
+    ulonglong2* const clear = (ulonglong2*)(SMEM ? s_slots : slots);
+    for (uint32_t i = threadIdx.x; i < cap / 2; i += blockDim.x) clear[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
     if (threadIdx.x < 4) counters[threadIdx.x] = 0;
     __syncthreads();
     uint32_t ins = 0, dup = 0, bad = 0;
-    ht_insert_rows(slots, log2cap, keys, payload, threadIdx.x, blockDim.x, n, preds, ins, dup, bad);
-    ht_count(ins, dup, bad, counters);
+    ht_insert_rows(SMEM ? s_slots : slots, log2cap, keys, payload, threadIdx.x, blockDim.x, n, preds, ins, dup, bad);
+    ht_count(ins, dup, bad, counters);  // ends with the table complete
+    if (SMEM)
+        for (uint32_t i = threadIdx.x; i < cap / 2; i += blockDim.x) ((ulonglong2*)slots)[i] = ((ulonglong2*)s_slots)[i];
 }
 
 // Smallest and largest key of the rows that pass the predicates (range[0],
@@ -1586,7 +1595,22 @@ gx_status gx_hashtable_build(gx_hashtable* ht, const int32_t* keys_dev, const in
     if (ht->layout == GX_HT_DENSE) return hashtable_build_dense(ht, keys_dev, payload_dev, n, bp, grid, s);
     const uint64_t cap = 1ull << ht->log2cap;
     if (ht->layout == GX_HT_LINEAR && cap <= kSmallHtSlots && n <= kSmallHtRows) {
-        ht_build_small_kernel<<<1, 1024, 0, s>>>(ht->slots, ht->log2cap, keys_dev, payload_dev, n, bp, ht->counters);
+        if (cap <= kSmemHtSlots) {
+            static bool attr_set[kMaxDevices] = {false};
+            int dev = 0;
+            cudaGetDevice(&dev);
+            if (!device_index_ok(dev)) return set_error(GX_ERR_INVALID, "device %d out of range", dev);
+            if (!attr_set[dev]) {
+                const gx_status st = allow_smem(ht_build_small_kernel<true>, 8 * kSmemHtSlots);
+                if (st) return st;
+                attr_set[dev] = true;
+            }
+            ht_build_small_kernel<true><<<1, 1024, 8 * cap, s>>>(ht->slots, ht->log2cap, keys_dev, payload_dev, n, bp,
+                                                                 ht->counters);
+        } else {
+            ht_build_small_kernel<false><<<1, 1024, 0, s>>>(ht->slots, ht->log2cap, keys_dev, payload_dev, n, bp,
+                                                            ht->counters);
+        }
         GX_CK(cudaGetLastError());
         return GX_OK;
     }

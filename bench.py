@@ -1121,7 +1121,12 @@ def main():
         if rank != 0:
             return
         from golap_public_b200 import queries
+        from oracle import oracle as O
 
+        if not O.ref_available():
+            print(json.dumps({"impl": "reference", "unavailable": "the reference tree was absent when the harness "
+                                                                  "was to be built"}))
+            return
         f, dd = make_data(args.seed)
         fact = queries.encode_fact(f, {"date_key": "cascaded"}, ROWS_PER_CHUNK, ROWS_PER_BLOCK, args.segments,
                                    residency=None)
@@ -1150,6 +1155,10 @@ def main():
         dist.init_process_group("nccl", timeout=timedelta(seconds=300))
     line, ctx = gpu_arm(args, rank, world)
     pk, pk_kind = peaks()
+    if not args.no_cpu:
+        from oracle import oracle as O
+
+        args.no_cpu = not O.ref_available()  # no harness without the reference tree: the GPU figures alone
     if rank == 0 and not args.no_cpu:
         cb = cpu_baseline(ctx["fact"], ctx["dd"], steps=3, warmup=1)
         line["cpu_baseline"] = {k: cb[k] for k in ("value", "unit", "cores", "kind", "sample", "ms")}

@@ -78,7 +78,6 @@ constexpr uint32_t kWsHead = 32 * 8 + 8 * 8 + 2 * GX_MAX_STEPS + 32 + 4;
 // four words of padding after each; the staged compressed bytes of a tile
 // (less than 7/8 of its rows' bytes, and the ends of the aligned copy)
 constexpr uint32_t kWsLaneShift0 = 5, kWsLaneShift1 = 7;
-constexpr uint32_t kWsLaneWords = kWsTile + (kWsTile >> kWsLaneShift0) * 4;
 constexpr uint32_t kWsStageWords = kWsTile * 7 / 8 + 16;
 static_assert(4 * kWsStageWords >= 4 * kWsTile * 7 / 8 + 38 && kWsStageWords % 4 == 0, "a staged range fits");
 constexpr uint32_t kWsQueueWords = (kWsBatch + 32) * 3;  // grouped plans: the warp's WsQueue, before its decode buffers
@@ -864,7 +863,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
 #pragma unroll
         for (uint32_t s = 0; s < NS; ++s) {
             src[s] = FLAT ? cols[Q.steps[s].col].src + (a + 4 * lane) * 4 : nullptr;
-            if (s >= PE && ((SIG >> (7 + 4 * s)) & kWkF) && Q.steps[s].lo > Q.steps[s].hi) some = 0;
+            if (s + 1 > PE && ((SIG >> (7 + 4 * s)) & kWkF) && Q.steps[s].lo > Q.steps[s].hi) some = 0;
         }
     }
 #pragma unroll 1

@@ -46,12 +46,12 @@
 // warps per SM and two row groups of loads in flight per warp.  Staging tiles
 // in shared memory held the kernel at 12 warps, waiting for its own copies:
 // 180 us; rows read in place, decisions in shared memory instead of registers,
-// row masks as predicates (1,400 -> 900 instructions per tile): 132 us.  The
+// row masks as predicates (1,450 -> 1,115 instructions per tile): 132 us.  The
 // star joins are bound by random table reads; there one row group per warp,
 // chains walked for all of a lane's rows together and dense group-table adds
 // took the 200M-row join from 6.3 to 2.2 ms, the four-join profit query over
 // 24M rows from 1.65 ms to 0.56 ms.  All-cascaded Q1 over 16M rows, values
-// unpacked in registers instead of through a decode buffer: 628 -> 205 us.
+// unpacked in registers instead of through a decode buffer: 626 -> 222 us.
 
 constexpr uint32_t kWsLog2 = 10;
 constexpr uint32_t kWsTile = 1u << kWsLog2;    // rows of one warp tile

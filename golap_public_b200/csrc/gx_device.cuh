@@ -310,12 +310,15 @@ __device__ __forceinline__ uint32_t lds32u(uint32_t a) {
 // header's token and offset are read at once (the offset's place follows from
 // the token), conditions are combined without branches, and literal and match
 // words take one path, so that the lanes stay together.  Length extensions of
-// more than two bytes cannot occur in a segment of at most 128 words.
+// more than two bytes: a match ends in its segment of at most 128 words and has
+// none; literals of more than 131 words go on past the segment, which ends in
+// them, so that they are left to the end (read in the loop, they cost it 2 %).
 __device__ __forceinline__ bool lz4_seg_lane(uint32_t p, uint32_t hi, uint32_t block_end, uint32_t info, uint32_t K,
                                              uint32_t out, bool active) {
     uint32_t L = 0, M = 0;      // literal and match words left of the sequence
     uint32_t lp = p, src = out; // where they are
     uint32_t bad = p > hi ? 1u : 0u;
+    constexpr uint32_t kLong = 1u << 31;  // a literal run of more words than the segment has left
     // the match of a sequence whose token nibble is mn and whose literals end at
     // q, L words from output word k on; p = the next token
     auto match = [&](uint32_t q, uint32_t mn, uint32_t k) {
@@ -352,7 +355,7 @@ __device__ __forceinline__ bool lz4_seg_lane(uint32_t p, uint32_t hi, uint32_t b
                 const uint32_t e = (x >> 8) & 255u, f = e == 255u ? (x >> 16) & 255u : 0u;
                 lit += e + f;
                 q += e == 255u ? 2u : 1u;
-                bad |= f == 255u ? 1u : 0u;
+                bad |= f == 255u ? kLong : 0u;
             }
             lp = q;
             L = min(lit >> 2, K - k);
@@ -377,6 +380,17 @@ __device__ __forceinline__ bool lz4_seg_lane(uint32_t p, uint32_t hi, uint32_t b
             }
             run = k < K;
         }
+    }
+    if (bad & kLong) {  // the segment ends in it: the rest of its length, then words to the end
+        uint32_t lit = 15 + 255 + 255, f = 255;
+        while (f == 255u && lp < hi) {
+            f = lds32u(lp) & 255u;
+            lit += f;
+            ++lp;
+        }
+        bad = (f == 255u ? 1u : 0u) | (lit & 3u) | (lp + 4 * (K - k) > hi ? 1u : 0u);
+        if (!bad)
+            for (; k < K; ++k, lp += 4, out += 4) sts32(out, lds32u(lp));
     }
     return !active || bad == 0;
 }

@@ -732,13 +732,12 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
     const uint32_t decs = (__ballot_sync(0xFFFFFFFFu, dec) >> sh) & m0;
     const uint32_t mixes = (__ballot_sync(0xFFFFFFFFu, mixed) >> sh) & m0;
     if (s == 0 && ((vm >> q) & 1u)) {
-        uint32_t f = cst | (decs ? kWsDecode : 0u) | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
-        if (SIG != 0 && bads) {
-            // a digit out of range is an error unless a constant step before it drops
-            // the rows; the run-time evaluator raises it only for rows alive at the step
-            if ((fails & ((1u << (__ffs(bads) - 1)) - 1u)) == 0) raise_error(kErrInvalid);
-            f |= kWsDead;
-        }
+        uint32_t f = cst | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
+        // a digit out of range is an error for rows alive at its step, which a
+        // step over rows before it may have dropped: unless a constant step
+        // before it drops the tile, its steps are all taken row by row
+        if (SIG != 0 && bads && (fails & ((1u << (__ffs(bads) - 1)) - 1u)) == 0) f = kWsMixed;
+        f |= decs ? kWsDecode : 0u;
         tiles[q].steps = f;
     }
     __syncwarp();

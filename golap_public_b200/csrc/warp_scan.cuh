@@ -693,15 +693,15 @@ __device__ constexpr bool ws_loose_step(uint32_t s, uint32_t n_steps, bool probe
 // The steps over columns that hold one value on their tile, decided once per
 // tile and for all tiles of the round together (their probes are one chain of
 // loads): lane (q << cl) + s decides step s of tile q, leaves its group-key
-// digit in sdig[lane] (kWsNone: out of range) and tiles[q].steps says which
-// steps are constant and whether one of them drops every row.
+// digit in sdig[lane] and tiles[q].steps says which steps are constant and
+// whether one of them drops every row.
 template <uint32_t SIG>
 __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, WsTile* tiles, const WsCol* cols,
                                                const uint64_t* whdr, uint32_t* sdig, uint64_t pol_keep,
                                                uint32_t lane) {
     const ShQuery& Q = P.q;
     const uint32_t cl = P.col_log2, q = lane >> cl, s = lane & ((1u << cl) - 1u);
-    bool isc = false, ok = true, bad = false, mixed = false, dec = false;
+    bool isc = false, ok = true, bad = false, mixed = false, dec = false, digits = false;
     if (((vm >> q) & 1u) && s < P.n_cols) {  // as a column
         const uint32_t m = cols[lane].mode;
         dec = m == kWmLz4 || m == kWmCasc || m == kWmBad;
@@ -721,22 +721,27 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
             if (ok && st.digit_card) {
                 const uint32_t dgt = (uint32_t)(pp - st.digit_base);
                 bad = dgt >= st.digit_card;
-                sdig[lane] = bad ? kWsNone : dgt;
+                sdig[lane] = dgt;
             }
         }
+        digits = bad || (SIG == 0 && !isc && st.digit_card);
     }
     const uint32_t m0 = (1u << (1u << cl)) - 1u, sh = q << cl;
     const uint32_t cst = (__ballot_sync(0xFFFFFFFFu, isc) >> sh) & m0;
     const uint32_t fails = (__ballot_sync(0xFFFFFFFFu, isc && !ok) >> sh) & m0;
     const uint32_t bads = (__ballot_sync(0xFFFFFFFFu, bad) >> sh) & m0;
+    const uint32_t digs = (__ballot_sync(0xFFFFFFFFu, digits) >> sh) & m0;
     const uint32_t decs = (__ballot_sync(0xFFFFFFFFu, dec) >> sh) & m0;
     const uint32_t mixes = (__ballot_sync(0xFFFFFFFFu, mixed) >> sh) & m0;
     if (s == 0 && ((vm >> q) & 1u)) {
         uint32_t f = cst | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
-        // a digit out of range is an error for rows alive at its step, which a
-        // step over rows before it may have dropped: unless a constant step
-        // before it drops the tile, its steps are all taken row by row
-        if (SIG != 0 && bads && (fails & ((1u << (__ffs(bads) - 1)) - 1u)) == 0) f = kWsMixed;
+        // a digit out of range is an error for rows alive at its step: its tile's
+        // steps are taken row by row (a step over rows before it may have dropped
+        // them) unless a constant step before it drops the tile.  Run-time plans
+        // also look at the digits of rows before they let a constant step drop
+        // them; the compile-time ones leave such a tile unread
+        const uint32_t before = fails ? (1u << (__ffs(fails) - 1)) - 1u : m0;
+        if (((fails ? digs : bads) & before) != 0) f = kWsMixed;
         f |= decs ? kWsDecode : 0u;
         tiles[q].steps = f;
     }
@@ -936,11 +941,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
             if ((K & kWkP) && !decided) m = ht_probe_rows<R>(stp.ht, stp.ht_log2, stp.ht_layout, s_hdr[s], v, m, pp, pol_keep);
             if (K & kWkD) {
                 const uint32_t dcard = stp.digit_card, dbase = (uint32_t)stp.digit_base, cdig = sdig[s];
-                if (decided) {  // (run-time form: kWsNone, a digit out of range)
-                    if (SIG == 0 && cdig >= dcard && m) {
-                        raise_error(kErrInvalid);
-                        m = 0;
-                    }
+                if (decided) {
 #pragma unroll
                     for (uint32_t r = 0; r < R; ++r) g[r] = g[r] * dcard + cdig;
                 } else {

@@ -1,6 +1,6 @@
 """Group-key digits out of range are an error for rows that are alive at their
-step, and only for those -- also where the column holds one value on a tile and
-is decided for all of its rows at once."""
+step, and only for those -- also where the column, or another step's, holds one
+value on a tile and is decided for all of its rows at once."""
 import numpy as np
 import pytest
 
@@ -79,3 +79,30 @@ def test_digit_of_a_constant_column(cuda, kind, codec, form):
             api.scan_check()
         assert e.value.status == L.GX_ERR_INVALID
         drop[at] = True
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("digit", ["rows", "constant"])
+def test_digit_before_a_constant_step_that_drops_the_tile(cuda, digit, form):
+    # the digit's step comes first: its rows are alive there, whatever a later step does to the tile
+    api.set_scan_form(form)
+    col = lambda v, c: api.Column(v.astype(np.int32), c, rows_per_chunk=5 * T, rows_per_block=T).to_device()
+    day = np.repeat(np.arange(8), T)
+    cd, cv = col(day, "cascaded"), col(np.ones(N), "none")
+    for last, bad in ((5, False), (6, True)):
+        k = np.where(day == 3, last, 2) if digit == "constant" else np.full(N, 2)
+        if digit == "rows":
+            k[np.arange(N) % 2 == 0] = 4
+            k[3 * T + 77] = last
+        agg = api.HashAggregate(64)
+        p = api.ScanPlan(agg=L.GX_AGG_SUM, groupby=agg)
+        p.group(col(k, "cascaded" if digit == "constant" else "none"), 0, 6).filter(cd, 4, 7).value(cv)
+        p.launch()
+        if bad:
+            with pytest.raises(L.GxError) as e:
+                api.scan_check()
+            assert e.value.status == L.GX_ERR_INVALID
+        else:
+            api.scan_check()
+            m = day >= 4
+            assert agg.read() == {int(g): int((k[m] == g).sum()) for g in np.unique(k[m])}

@@ -1913,7 +1913,8 @@ static gx_status ensure_kernel_attrs() {
     if (!st) st = allow_smem(shared_scan_kernel<1024, 1>, sh_max);
     if (!st) st = allow_smem(shared_scan_kernel<kShSingleNT, 4, true>, sh_max);
     if (!st) st = allow_smem(pipe_scan_kernel, kPipeMaxDynSmem);
-    if (!st) st = allow_smem(warp_scan_kernel<0>, kWsMaxDynSmem);
+    if (!st) st = allow_smem(warp_scan_kernel<kSigRt>, kWsMaxDynSmem);
+    if (!st) st = allow_smem(warp_scan_kernel<kSigRtGroup>, kWsMaxDynSmem);
     if (!st) st = allow_smem(warp_scan_kernel<kSigQ1>, kWsMaxDynSmem);
     if (!st) st = allow_smem(warp_scan_kernel<kSigQ2>, kWsMaxDynSmem);
     if (!st) st = allow_smem(warp_scan_kernel<kSigQ3>, kWsMaxDynSmem);
@@ -2420,7 +2421,7 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
     const uint32_t sig = plan->n_steps <= 6 ? ws_sig(plan->n_steps, P.q.agg, P.q.grouped != 0, kinds[0], kinds[1],
                                                      kinds[2], kinds[3], kinds[4], kinds[5])
                                             : 0u;
-    void (*kern)(WsParams) = warp_scan_kernel<0>;
+    void (*kern)(WsParams) = P.q.grouped ? warp_scan_kernel<kSigRtGroup> : warp_scan_kernel<kSigRt>;
     if (sig == kSigQ1) kern = warp_scan_kernel<kSigQ1>;
     else if (sig == kSigQ2) kern = warp_scan_kernel<kSigQ2>;
     else if (sig == kSigQ3) kern = warp_scan_kernel<kSigQ3>;

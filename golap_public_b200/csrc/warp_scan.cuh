@@ -683,6 +683,12 @@ __device__ __forceinline__ bool ws_probe1(const ShStep& st, uint64_t hdr, int32_
     return true;
 }
 
+// Plans of no known signature (below) are evaluated at run time: their
+// "signatures" have no step count, and bit 6 for those with a group key.
+constexpr uint32_t kSigRt = 0, kSigRtGroup = 1u << 6;
+template <uint32_t SIG>
+constexpr bool kWsRunTime = (SIG & 7) == 0;
+
 // Steps whose column need not be direct in the flat evaluator (constant, of
 // two runs or decoded will do): probes and the first step, when they neither
 // carry nor are the last.
@@ -724,7 +730,7 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
                 sdig[lane] = dgt;
             }
         }
-        digits = bad || (SIG == 0 && !isc && st.digit_card);
+        digits = bad || (SIG == kSigRtGroup && !isc && st.digit_card);
     }
     const uint32_t m0 = (1u << (1u << cl)) - 1u, sh = q << cl;
     const uint32_t cst = (__ballot_sync(0xFFFFFFFFu, isc) >> sh) & m0;
@@ -751,7 +757,7 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
 // ---- plan signatures: compile-time evaluators for the known query shapes
 // A signature packs the step count (bits 0-2), the aggregate (3-5), grouped
 // (6) and per step s a kind nibble at bit 7 + 4 s: 1 FILTER, 2 PROBE,
-// 4 CARRY, 8 group-key digit.  Signature 0 is the run-time evaluator.
+// 4 CARRY, 8 group-key digit.
 constexpr uint32_t kWkF = 1, kWkP = 2, kWkC = 4, kWkD = 8;
 constexpr uint32_t ws_sig(uint32_t ns, uint32_t agg, bool grouped, uint32_t k0, uint32_t k1 = 0, uint32_t k2 = 0,
                           uint32_t k3 = 0, uint32_t k4 = 0, uint32_t k5 = 0) {
@@ -840,7 +846,7 @@ __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
 // mask.  A compile-time signature loads all columns of the batch before any
 // is used and unrolls its steps: up to the last probe step by step, the
 // filters after it and the aggregate row by row, where a row's mask is a
-// predicate.  The run-time form (SIG 0) loads a column at its step.  FLAT:
+// predicate.  Run-time plans with a group key load a column at its step.  FLAT:
 // [a, b) is whole batches and every column is direct or a loose step's that is
 // not packed (a sorted date), so that a batch's loads are unconditional and all
 // in flight together.  Steps over constant columns were decided by
@@ -852,18 +858,18 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
                                            uint32_t a, uint32_t b, uint32_t* tkey, WsQueue* wq, uint32_t& qn,
                                            uint64_t pol_keep, const uint64_t* s_hdr,
                                            uint32_t lane) {
-    constexpr bool GR = SIG == 0 || ((SIG >> 6) & 1) != 0;  // may be grouped: the queue holds one row group
+    constexpr bool RT = kWsRunTime<SIG>;
+    constexpr bool GR = ((SIG >> 6) & 1) != 0;  // grouped: the queue holds one row group
     constexpr uint32_t H = GR ? 1 : kWsEvalGroups;
     constexpr uint32_t R = 4 * H;
-    constexpr uint32_t NS = SIG ? (SIG & 7) : 1;
-    constexpr uint32_t PE = SIG ? kWsProbesEnd<SIG> : 0;  // steps [0, PE) run step by step
-    const uint32_t ns = SIG ? NS : Q.n_steps;
-    const uint32_t agg = SIG ? (SIG >> 3) & 7 : Q.agg;
-    const bool grouped = SIG ? ((SIG >> 6) & 1) != 0 : Q.grouped != 0;
+    constexpr uint32_t NS = RT ? 1 : (SIG & 7);
+    constexpr uint32_t PE = RT ? 0 : kWsProbesEnd<SIG>;  // steps [0, PE) run step by step
+    const uint32_t ns = RT ? Q.n_steps : NS;
+    const uint32_t agg = RT ? Q.agg : (SIG >> 3) & 7;
     int64_t acc = 0;
     const uint8_t* src[NS];  // FLAT: the lane's quad of each step's column
     uint32_t some = ~0u;     // signatures: 0 when a filter after the probes has an empty range
-    if (SIG) {
+    if (!RT) {
 #pragma unroll
         for (uint32_t s = 0; s < NS; ++s) {
             src[s] = FLAT ? cols[Q.steps[s].col].src + (a + 4 * lane) * 4 : nullptr;
@@ -884,7 +890,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
         uint32_t g[R], carry[R];
 #pragma unroll
         for (uint32_t r = 0; r < R; ++r) g[r] = carry[r] = 0;
-        if (SIG) {
+        if (!RT) {
             // (values of rows that are not wanted are not used: any will do.  A quad with one
             // wanted row ends at most 12 bytes after its block, inside the payload)
 #pragma unroll
@@ -964,7 +970,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
             }
         };
         uint32_t val[R];  // the last column
-        if constexpr (SIG != 0) {
+        if constexpr (!RT) {
 #pragma unroll
             for (uint32_t s = 0; s < NS; ++s) {
                 const uint32_t K = (SIG >> (7 + 4 * s)) & 15u;
@@ -999,7 +1005,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
         // the filters after the probes and the aggregate, row by row
         auto kept = [&](uint32_t r) {
             bool k = ((m >> r) & 1u) != 0;
-            if (SIG) {
+            if (!RT) {
 #pragma unroll
                 for (uint32_t s = PE; s < NS; ++s)
                     if ((SIG >> (7 + 4 * s)) & kWkF) {
@@ -1016,7 +1022,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
                    : agg == GX_AGG_COUNT     ? 1
                                              : (int64_t)x;
         };
-        if (!grouped) {
+        if (!GR) {
 #pragma unroll
             for (uint32_t r = 0; r < R; ++r) {
                 if constexpr (SIG == kSigQ1) {
@@ -1058,6 +1064,114 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
     return acc;
 }
 
+// A run-time plan without a group key over tile rows [a, b), step by step: a
+// step issues the loads of four quads (512 rows of the warp) together, those of
+// rows still kept, and leaves the rows it keeps in a mask (bit 4 j + i: row
+// 128 j + 4 lane + i); probes go two quads at a time, and a carried column is
+// read again beside the last step's.  What kind of step it is, how its column
+// is read and the aggregate are so decided once per 512 rows: row group by row
+// group (as ws_eval takes grouped plans, whose keys live in registers) these
+// decisions and one load in flight per step bound the scan: over 20M rows a sum
+// 91 us, a filtered sum 144 us, a date probe with a filter and a sum 174 us;
+// 21, 38 and 54 us here.  Returns the lane's part of the sum.
+__device__ __forceinline__ int64_t ws_eval_steps(const ShQuery& Q, const WsCol* cols, uint32_t cst, uint32_t a,
+                                                 uint32_t b, uint64_t pol_keep, const uint64_t* s_hdr,
+                                                 uint32_t lane) {
+    uint32_t keep = ~0u;
+    if (a != 0 || b != kWsTile) {
+        keep = 0;
+        for (uint32_t j = a / kWsBatch; j * kWsBatch < b; ++j) {
+            const uint32_t row = j * kWsBatch + 4 * lane, n = row < b ? min(4u, b - row) : 0u;
+            keep |= ((1u << n) - 1u) << (4 * j);
+        }
+    }
+    // quads j .. j + 3 of a column (those with a row kept)
+    auto load = [&](const WsCol& d, uint32_t j, uint32_t k, uint32_t (&x)[16]) {
+        const uint32_t row = j * kWsBatch + 4 * lane;
+        if (d.mode == kWmDirect) {
+            const uint8_t* p = d.src + 4 * row;
+#pragma unroll
+            for (uint32_t h = 0; h < 4; ++h)
+                if ((k >> (4 * h)) & 15u) ws_put(x, h, ws_ld_rows(p + 4 * kWsBatch * h));
+        } else {
+#pragma unroll
+            for (uint32_t h = 0; h < 4; ++h)
+                if ((k >> (4 * h)) & 15u) ws_put(x, h, ws_quad(d, row + kWsBatch * h));
+        }
+    };
+    const uint32_t ns = Q.n_steps, agg = Q.agg, j_end = (b + kWsBatch - 1) / kWsBatch;
+    const WsCol* carried = nullptr;
+    int64_t acc = 0;
+#pragma unroll 1
+    for (uint32_t s = 0; s < ns; ++s) {
+        const ShStep& stp = Q.steps[s];
+        const WsCol& d = cols[stp.col];
+        const uint32_t f = stp.flags;
+        const bool last = s + 1 == ns, decided = ((cst >> s) & 1u) != 0;
+        if (f & GX_STEP_CARRY) carried = &d;
+        const bool filt = (f & GX_STEP_FILTER) && !decided;
+        if (filt && stp.lo > stp.hi) return 0;
+        const uint32_t lo = (uint32_t)stp.lo, span = (uint32_t)stp.hi - lo;
+        if ((f & GX_STEP_PROBE) && !decided) {
+#pragma unroll 1
+            for (uint32_t j = a / kWsBatch; j < j_end; j += 2) {
+                uint32_t k = (keep >> (4 * j)) & 255u, m = k;
+                if (!__any_sync(0xFFFFFFFFu, k)) continue;
+                uint32_t v[8], pay[8];
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h)
+                    if ((k >> (4 * h)) & 15u) ws_put(v, h, ws_quad(d, (j + h) * kWsBatch + 4 * lane));
+                if (filt) {
+#pragma unroll
+                    for (uint32_t r = 0; r < 8; ++r)
+                        if (v[r] - lo > span) m &= ~(1u << r);
+                }
+                m = ht_probe_rows<8>(stp.ht, stp.ht_log2, stp.ht_layout, s_hdr[s], v, m, pay, pol_keep);
+                keep &= ~((k & ~m) << (4 * j));
+            }
+        }
+        const bool here = filt && !(f & GX_STEP_PROBE);
+        if (here || last) {
+            const bool both = agg == GX_AGG_SUM_PRODUCT || agg == GX_AGG_SUM_DIFF;
+#pragma unroll 1
+            for (uint32_t j = a / kWsBatch; j < j_end; j += 4) {
+                uint32_t k = (keep >> (4 * j)) & 0xFFFFu;
+                if (!__any_sync(0xFFFFFFFFu, k)) continue;
+                uint32_t x[16], c[16];
+                if (here || agg != GX_AGG_COUNT) load(d, j, k, x);
+                if (last && both) load(*carried, j, k, c);
+                if (here) {
+                    uint32_t m = k;
+#pragma unroll
+                    for (uint32_t r = 0; r < 16; ++r)
+                        if (x[r] - lo > span) m &= ~(1u << r);
+                    keep &= ~((k & ~m) << (4 * j));
+                    k = m;
+                }
+                if (!last) continue;
+                if (agg == GX_AGG_SUM_PRODUCT) {
+#pragma unroll
+                    for (uint32_t r = 0; r < 16; ++r)
+                        if ((k >> r) & 1u) acc += (int64_t)(int32_t)x[r] * (int32_t)c[r];
+                } else if (agg == GX_AGG_COUNT) {
+                    acc += __popc(k);
+                } else {
+#pragma unroll
+                    for (uint32_t r = 0; r < 16; ++r)
+                        if ((k >> r) & 1u) acc += (int32_t)x[r];
+                    if (agg == GX_AGG_SUM_DIFF) {
+#pragma unroll
+                        for (uint32_t r = 0; r < 16; ++r)
+                            if ((k >> r) & 1u) acc -= (int32_t)c[r];
+                    }
+                }
+            }
+        }
+        if (!__any_sync(0xFFFFFFFFu, keep)) break;
+    }
+    return acc;
+}
+
 // The general evaluator out of line: ragged tiles, columns that are not
 // direct, run-time plans.
 template <uint32_t SIG>
@@ -1074,13 +1188,18 @@ __device__ __noinline__ int64_t ws_eval_any(const ShQuery& Q, const WsCol* cols,
 // CTAs per SM each form is built for.  Scalar signatures (two row groups and
 // their columns in registers) keep 96 registers: five CTAs, 20 warps, scan Q1
 // over 60M rows in 132 us where four take 165 us (too few loads in flight) and
-// six 150 us (spills).  Grouped ones (one row group, probes) take six: the
-// 200M-row star join 2.17 ms, 2.26 with five, 2.35 with seven; more shared
-// memory costs them L1, which holds their reads in flight: 2048 group slots
-// instead of 512, 4.2 ms).  The group-by without joins and run-time plans wait
-// on group-table adds and take eight (30M rows into 1.4M groups: 585 us, 674
-// with six; as a run-time plan 782).
-constexpr int ws_ctas(uint32_t sig) { return sig == 0 || sig == kSigGroup ? 8 : ((sig >> 6) & 1) ? 6 : 5; }
+// six 150 us (spills); scalar run-time plans likewise (a filtered sum over 20M
+// rows 38 us, with four 43, with six 38 but a pruned one 13.7 for 12.6).
+// Grouped ones (one row group, probes) take six: the 200M-row star join 2.17 ms,
+// 2.26 with five, 2.35 with seven; more shared memory costs them L1, which holds
+// their reads in flight: 2048 group slots instead of 512, 4.2 ms).  The group-by
+// without joins waits on group-table adds and takes eight (30M rows into 1.4M
+// groups: 585 us, 674 with six; as a run-time plan 782).  Grouped run-time plans
+// take seven (20M rows counted into 50 groups 171 us, with eight 195; summed into
+// 550 groups 468 us, 488 with eight and 502 with six).
+constexpr int ws_ctas(uint32_t sig) {
+    return sig == kSigGroup ? 8 : sig == kSigRtGroup ? 7 : ((sig >> 6) & 1) ? 6 : 5;
+}
 
 template <uint32_t SIG>
 __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __grid_constant__ WsParams P) {
@@ -1218,9 +1337,11 @@ __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __
             if (!(st & kWsDead)) {
                 // whole row batches of direct columns: the flat form
                 const uint32_t* const dig = wdig + (q << cl);
-                if (SIG != 0 && !(st & kWsMixed) && ((T.b - T.a) & (kWsPartRows - 1u)) == 0)
-                    local += ws_eval<SIG, SIG != 0>(Q, cols, st, dig, T.a, T.b, tkey, wq, qn, pol_keep, whdr,
-                                                     lane);
+                if constexpr (SIG == kSigRt)
+                    local += ws_eval_steps(Q, cols, st, T.a, T.b, pol_keep, whdr, lane);
+                else if (!kWsRunTime<SIG> && !(st & kWsMixed) && ((T.b - T.a) & (kWsPartRows - 1u)) == 0)
+                    local += ws_eval<SIG, !kWsRunTime<SIG>>(Q, cols, st, dig, T.a, T.b, tkey, wq, qn, pol_keep, whdr,
+                                                            lane);
                 else
                     local += ws_eval_any<SIG>(Q, cols, st, dig, T.a, T.b, tkey, wq, &qn, pol_keep, whdr, lane);
             }

@@ -139,17 +139,86 @@ __device__ __forceinline__ bool lz4_len_ext(const uint32_t* __restrict__ A, uint
     }
 }
 
-// Decodes one segment of a segmented LZ4 block per group of G lanes (G a power
-// of two <= 32, a group's lanes adjacent; gl = this lane's index in it), the
-// groups of a warp in step: one sequence each per round.  Called by whole
-// warps; lanes of a group without a segment pass active = false.  Every lane
-// of a group parses the same sequence headers (broadcast loads); literal runs
-// and matches are copied G words per step.  A match's words are all computed
-// from output before the match: out[k + i] = out[k - offw + (i mod offw)] (LZ4
-// overlap semantics), so the barrier before each match orders it after every
-// earlier write of the group.  A = the words from byte wbase (staged, or in
-// place), [lo, hi) the tile's compressed range, K output words.  Returns 0 or
-// kErrCorrupt (the same for every lane of a group).
+// Decodes one segment of a segmented LZ4 block with a group of G lanes
+// (G a power of two <= 32, the group's lanes adjacent in one warp; gmask =
+// the group's lanes, gl = this lane's index in the group).  Every lane of the
+// group parses the same sequence headers (broadcast shared loads), so the
+// group stays converged; literal runs and matches are copied G words per
+// step.  A match's words are all computed from output before the match:
+// out[k + i] = out[k - offw + (i mod offw)] (LZ4 overlap semantics), so one
+// __syncwarp before each match orders it after every earlier write of the
+// group.  A = the words from byte wbase (staged, or in place), [lo, hi) the
+// tile's compressed range, K output words.  Returns 0 or kErrCorrupt (the same
+// for every lane of the group).
+__device__ __forceinline__ int lz4_seg_group(const uint32_t* __restrict__ A, uint32_t wbase, uint32_t lo,
+                                             uint32_t hi, uint32_t block_end, uint32_t comp_pos, uint32_t info,
+                                             uint32_t K, uint32_t* __restrict__ out, uint32_t gl, uint32_t G,
+                                             uint32_t gmask) {
+    if (comp_pos < lo || comp_pos > hi) return kErrCorrupt;
+    uint32_t pos = comp_pos, k = 0, litw = 0, mnib = 0;
+    bool tok_next = true;
+    if (info & 16u) {  // the segment starts inside a sequence
+        const uint32_t lit = info >> 5;
+        if (lit & 3u) return kErrCorrupt;
+        litw = lit >> 2;
+        mnib = info & 15u;
+        tok_next = false;
+    }
+    while (true) {
+        if (tok_next) {
+            if (k >= K) break;
+            if (pos >= hi) return kErrCorrupt;
+            const uint32_t x = fetch4(A, pos - wbase);
+            uint32_t lit = (x >> 4) & 15u;
+            mnib = x & 15u;
+            ++pos;
+            if (lit == 15 && !lz4_len_ext(A, wbase, pos, hi, lit)) return kErrCorrupt;
+            if (lit & 3u) return kErrCorrupt;
+            litw = lit >> 2;
+        }
+        const uint32_t n = min(litw, K - k);
+        if ((uint64_t)pos + 4ull * n > hi) return kErrCorrupt;
+        {
+            const uint32_t r = pos - wbase, w = r >> 2, sh = (r & 3u) * 8;
+            for (uint32_t i = gl; i < n; i += G) out[k + i] = __funnelshift_r(A[w + i], A[w + i + 1], sh);
+        }
+        k += n;
+        pos += 4 * n;
+        if (k >= K) break;  // the segment ends inside or right after the literals
+        // literals done: the block may end here (then the segment is short)
+        if (pos == block_end || (uint64_t)pos + 2 > hi) return kErrCorrupt;
+        const uint32_t off = fetch4(A, pos - wbase) & 0xFFFFu;
+        pos += 2;
+        uint32_t ml = mnib + 4;
+        if (mnib == 15 && !lz4_len_ext(A, wbase, pos, hi, ml)) return kErrCorrupt;
+        if ((off & 3u) || (ml & 3u) || off == 0) return kErrCorrupt;
+        const uint32_t offw = off >> 2, mw = ml >> 2;
+        if (offw > k || mw > K - k) return kErrCorrupt;
+        __syncwarp(gmask);
+        const uint32_t* src = out + (k - offw);
+        if (offw >= mw) {
+            for (uint32_t i = gl; i < mw; i += G) out[k + i] = src[i];
+        } else if (offw == 1) {
+            const uint32_t v = src[0];
+            for (uint32_t i = gl; i < mw; i += G) out[k + i] = v;
+        } else {
+            uint32_t r = gl % offw;
+            const uint32_t step = G % offw;
+            for (uint32_t i = gl; i < mw; i += G) {
+                out[k + i] = src[r];
+                r += step;
+                if (r >= offw) r -= offw;
+            }
+        }
+        k += mw;
+        tok_next = true;
+    }
+    return 0;
+}
+
+// As lz4_seg_group, with the groups of a warp in step: one sequence each per
+// round, for columns of short sequences.  Called by whole warps; lanes of a
+// group without a segment pass active = false.
 // What bounds it: the chain of dependent instructions of a sequence (100 or
 // so, 6 to 8 cycles each with few warps resident), of which a segment of small
 // integers has nearly one per row.  A round of short sequences therefore reads
@@ -157,7 +226,8 @@ __device__ __forceinline__ bool lz4_len_ext(const uint32_t* __restrict__ A, uint
 // fetches the next token before the copy, and the groups stay in step (their
 // own loops drifted apart and ran one after another).  Q1 over 10M rows of such
 // columns 665 -> 570 us, decoding 24M discount rows 353 -> 330; a column known
-// to hold many short sequences takes lz4_seg_lane in the scan.
+// to hold many short sequences takes lz4_seg_lane in the scan.  Sequences longer
+// than such a round pay for looking (LzGroups below).
 __device__ __forceinline__ int lz4_seg_step(const uint32_t* __restrict__ A, uint32_t wbase, uint32_t lo, uint32_t hi,
                                             uint32_t block_end, uint32_t comp_pos, uint32_t info, uint32_t K,
                                             uint32_t* __restrict__ out, uint32_t gl, uint32_t G, bool active) {
@@ -280,6 +350,44 @@ __device__ __forceinline__ int lz4_seg_step(const uint32_t* __restrict__ A, uint
         __syncwarp();
     }
     return active && !ok ? kErrCorrupt : 0;
+}
+
+// Which of the two a column takes: groups in step (gx_dcol::lz4_steps) from three
+// sequences to 16 rows on.  Measured on both sides of that line, groups in step
+// against each on its own (time of decompressing / a pipelined / a shared scan
+// of 8M rows): 0.24 to 0.78 sequences per row 0.88 to 1.02 / 0.75 to 0.84 / 0.80
+// to 0.96; 0.02 to 0.13 per row 0.97 to 1.14 / 1.05 to 1.12 / 1.03 to 1.09.
+enum class LzGroups { kEither, kAlone, kInStep };  // the decoders an instance holds
+
+// nseg segments (block segments j0 ..; entries at seg) by the tid-th of NT
+// threads, 1 << glog lanes each, from the words A on; segment t goes to buf + t *
+// (seg_rows + pad).  Records an error in *err.  (Each decoder with a loop of its
+// own: with one loop around both, a shared scan of long sequences took 5 % more.)
+template <LzGroups LZ = LzGroups::kEither>
+__device__ __forceinline__ void lz4_segs(bool steps, uint32_t tid, uint32_t NT, uint32_t glog, uint32_t j0,
+                                         uint32_t nseg, uint32_t rows, uint32_t seg_rows,
+                                         const uint32_t* __restrict__ A, uint32_t wbase, uint32_t lo, uint32_t hi,
+                                         uint32_t block_end, const uint32_t* seg, uint32_t* buf, uint32_t pad,
+                                         int* err) {
+    const uint32_t G = 1u << glog, gl = tid & (G - 1u), lane = tid & 31u;
+    if (LZ == LzGroups::kInStep || (LZ == LzGroups::kEither && steps)) {
+        for (uint32_t t0 = (tid & ~31u) >> glog; t0 < nseg; t0 += (NT >> glog)) {  // whole warps go round together
+            const uint32_t t = t0 + (lane >> glog);
+            const bool in = t < nseg;
+            const uint32_t ts = in ? t : 0u, K = min(seg_rows, rows - (j0 + ts) * seg_rows);
+            const int r2 = lz4_seg_step(A, wbase, lo, hi, block_end, seg[2 * ts], seg[2 * ts + 1], K,
+                                        buf + ts * (seg_rows + pad), gl, G, in);
+            if (r2 && gl == 0) *err = r2;
+        }
+    } else {
+        const uint32_t gmask = G >= 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(G - 1u)));
+        for (uint32_t t = tid >> glog; t < nseg; t += (NT >> glog)) {
+            const uint32_t K = min(seg_rows, rows - (j0 + t) * seg_rows);
+            const int r2 = lz4_seg_group(A, wbase, lo, hi, block_end, seg[2 * t], seg[2 * t + 1], K,
+                                         buf + t * (seg_rows + pad), gl, G, gmask);
+            if (r2 && gl == 0) *err = r2;
+        }
+    }
 }
 
 // ---- one lane per segment, from staged bytes

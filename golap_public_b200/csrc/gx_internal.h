@@ -137,7 +137,7 @@ struct gx_dcol {
     uint32_t n_slots;           // n_chunks * blocks_per_chunk
     uint64_t payload_bytes;     // size of the payload allocation
     uint32_t host_mapped;       // payload lives in pinned host memory (no TMA staging)
-    uint32_t pad_;
+    uint32_t lz4_steps;         // LZ4 with segments: many short sequences (LzGroups in gx_device.cuh)
 };
 
 // Bit-packed stream reader: element i of width w (0..32).
@@ -228,6 +228,7 @@ struct gx_column {
         v.n_slots = n_slots;
         v.payload_bytes = host_pending ? dev_payload_bytes : payload.size();
         v.host_mapped = residency == 2 ? 1u : 0u;
+        v.lz4_steps = lz4_seqs * 16 >= n_rows * 3 ? 1u : 0u;
         return v;
     }
 };

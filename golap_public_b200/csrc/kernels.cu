@@ -206,7 +206,8 @@ __device__ __forceinline__ int stage_bytes(const gx_dcol& c, const uint8_t* src,
 // Returns the layout (kRows: buf[r]; kSegRows: buf[r + ((r >> seg_shift) <<
 // pad_log2)], each segment followed by 2^pad_log2 pad words) or -1 with
 // *s_err set.  All NT threads call it.
-template <int NT, int MAXT>
+// LZ: the LZ4 decoders the instance holds (both take more registers).
+template <int NT, int MAXT, LzGroups LZ = LzGroups::kEither>
 __device__ __forceinline__ int decode_tile(const gx_dcol& c, uint32_t slot, uint32_t rows, uint32_t r0, uint32_t n,
                                            uint32_t* buf, uint8_t* stage, uint64_t* mbar, uint32_t& phase,
                                            uint32_t* tmp, int* s_err, uint32_t& pad_log2, uint32_t* seg_smem) {
@@ -317,7 +318,7 @@ __device__ __forceinline__ int decode_tile(const gx_dcol& c, uint32_t slot, uint
                 __syncthreads();
                 return kRows;
             }
-            // a group of G adjacent lanes per segment; segment t at buf + t * (seg_rows + G)
+            // a group of G adjacent lanes per segment; segment t at buf + t * (seg_rows + pad)
             // lanes per segment: a whole warp when the tile is mostly literals
             // (few sequences; conflict-free 32-word copies), else spread the
             // segments over all NT threads
@@ -326,21 +327,11 @@ __device__ __forceinline__ int decode_tile(const gx_dcol& c, uint32_t slot, uint
             // 256 words every decode buffer reserves beyond its rows
             uint32_t glog = literal_tile ? 5u : seg_group_log2(nseg, NT);
             while (glog > 0 && glog < 5 && (nseg << glog) > 256u) --glog;
-            const uint32_t G = 1u << glog;
-            // pad words after each segment: G (groups of a warp on distinct
+            // pad words after each segment: as many as lanes (groups of a warp on distinct
             // banks), 1 for a whole-warp group (its stores are contiguous)
             const uint32_t pl = glog == 5 ? 0u : glog;
-            const uint32_t gl = tid & (G - 1u);
-            // (whole warps go round together)
-            for (uint32_t t0 = (tid & ~31u) >> glog; t0 < nseg; t0 += (NT >> glog)) {
-                const uint32_t t = t0 + ((tid & 31u) >> glog);
-                const bool in = t < nseg;
-                const uint32_t j = j0 + (in ? t : 0u), ts = in ? t : 0u;
-                const uint32_t K = min(seg_rows, rows - j * seg_rows);
-                const int r2 = lz4_seg_step((const uint32_t*)stage, wbase, lo, hi, d.comp_bytes, seg_smem[2 * ts],
-                                            seg_smem[2 * ts + 1], K, buf + ts * (seg_rows + (1u << pl)), gl, G, in);
-                if (r2 && gl == 0) *s_err = r2;
-            }
+            lz4_segs<LZ>(c.lz4_steps, tid, NT, glog, j0, nseg, rows, seg_rows, (const uint32_t*)stage, wbase, lo, hi,
+                         d.comp_bytes, seg_smem, buf, 1u << pl, s_err);
             pad_log2 = pl;
             __syncthreads();
             return kSegRows;
@@ -707,8 +698,12 @@ __global__ void __launch_bounds__(1024) batch_items_kernel(const QueryDesc* __re
 
 // Decompress tiles of slots [slot0, slot0 + gridDim.x / tpb) into dst, rows
 // laid out contiguously from the first row of chunk row0.  One CTA per tile.
-template <int NT, int MAXT>
-__global__ void __launch_bounds__(NT) decompress_kernel(const __grid_constant__ gx_dcol c, uint32_t slot0, uint32_t tile_rows,
+// The small form's shared memory lets six CTAs share an SM; with registers for
+// them (80) instead of the 48 the compiler picks by itself, 24M discount rows of
+// short sequences take 295 us instead of 337, and no instance spills (the stack
+// of one that did added 2 us to a launch of 17).
+template <int NT, int MAXT, LzGroups LZ>
+__global__ void __launch_bounds__(NT, MAXT == kTileRows ? 6 : 1) decompress_kernel(const __grid_constant__ gx_dcol c, uint32_t slot0, uint32_t tile_rows,
                                                         uint32_t tpb, uint64_t row0, int32_t* dst) {
     using C = Cfg<MAXT>;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -729,8 +724,8 @@ __global__ void __launch_bounds__(NT) decompress_kernel(const __grid_constant__ 
     }
     __syncthreads();
     uint32_t phase = 0, pad_log2 = 0;
-    const int layout = decode_tile<NT, MAXT>(c, slot, d.n_rows, r0, n, buf, stage, &s_mbar, phase, s_tmp, &s_err,
-                                             pad_log2, s_seg);
+    const int layout = decode_tile<NT, MAXT, LZ>(c, slot, d.n_rows, r0, n, buf, stage, &s_mbar, phase, s_tmp, &s_err,
+                                                 pad_log2, s_seg);
     if (s_err) {
         if (threadIdx.x == 0) raise_error(s_err);
         return;
@@ -1410,8 +1405,9 @@ gx_status gx_decompress_chunks(const gx_column* col, uint64_t first_chunk, uint6
     cudaGetDevice(&dev);
     if (!device_index_ok(dev)) return set_error(GX_ERR_INVALID, "device %d out of range", dev);
     if (!attr_set[dev]) {
-        gx_status st = allow_smem(decompress_kernel<128, kTileRows>, dec_smem_bytes<kTileRows>());
-        if (!st) st = allow_smem(decompress_kernel<256, kMaxRowsPerBlock>, dec_smem_bytes<kMaxRowsPerBlock>());
+        gx_status st = allow_smem(decompress_kernel<128, kTileRows, LzGroups::kAlone>, dec_smem_bytes<kTileRows>());
+        if (!st) st = allow_smem(decompress_kernel<128, kTileRows, LzGroups::kInStep>, dec_smem_bytes<kTileRows>());
+        if (!st) st = allow_smem(decompress_kernel<256, kMaxRowsPerBlock, LzGroups::kEither>, dec_smem_bytes<kMaxRowsPerBlock>());
         if (st) return st;
         attr_set[dev] = true;
     }
@@ -1421,12 +1417,16 @@ gx_status gx_decompress_chunks(const gx_column* col, uint64_t first_chunk, uint6
     const uint32_t tile = pick_tile_rows(&col, 1);
     const uint32_t tpb = (col->rows_per_block + tile - 1) / tile;
     cudaStream_t s = (cudaStream_t)stream;
-    if (tile <= kTileRows)
-        decompress_kernel<128, kTileRows><<<nslots * tpb, 128, dec_smem_bytes<kTileRows>(), s>>>(
-            col->view(), slot0, tile, tpb, row0, (int32_t*)dst_dev);
+    const gx_dcol v = col->view();
+    if (tile > kTileRows)
+        decompress_kernel<256, kMaxRowsPerBlock, LzGroups::kEither>
+            <<<nslots * tpb, 256, dec_smem_bytes<kMaxRowsPerBlock>(), s>>>(v, slot0, tile, tpb, row0, (int32_t*)dst_dev);
+    else if (v.lz4_steps)
+        decompress_kernel<128, kTileRows, LzGroups::kInStep>
+            <<<nslots * tpb, 128, dec_smem_bytes<kTileRows>(), s>>>(v, slot0, tile, tpb, row0, (int32_t*)dst_dev);
     else
-        decompress_kernel<256, kMaxRowsPerBlock><<<nslots * tpb, 256, dec_smem_bytes<kMaxRowsPerBlock>(), s>>>(
-            col->view(), slot0, tile, tpb, row0, (int32_t*)dst_dev);
+        decompress_kernel<128, kTileRows, LzGroups::kAlone>
+            <<<nslots * tpb, 128, dec_smem_bytes<kTileRows>(), s>>>(v, slot0, tile, tpb, row0, (int32_t*)dst_dev);
     GX_CK(cudaGetLastError());
     return GX_OK;
 }

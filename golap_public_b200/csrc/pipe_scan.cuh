@@ -243,18 +243,9 @@ __device__ __forceinline__ int pipe_lz4_tile(const gx_dcol& c, const PipeTile& T
     const bool literal_tile = (uint64_t)(pc.hi - pc.lo) * 8 >= (uint64_t)T.n * 4 * 7;
     uint32_t glog = literal_tile ? 5u : seg_group_log2(nseg, kPipeNC);
     while (glog > 0 && glog < 5 && (nseg << glog) > 256u) --glog;
-    const uint32_t G = 1u << glog;
     const uint32_t pl = glog == 5 ? 0u : glog;
-    const uint32_t gl = tid & (G - 1u);
-    for (uint32_t t0 = (tid & ~31u) >> glog; t0 < nseg; t0 += (kPipeNC >> glog)) {  // whole warps go round together
-        const uint32_t t = t0 + ((tid & 31u) >> glog);
-        const bool in = t < nseg;
-        const uint32_t ts = in ? t : 0u, j = j0 + ts;
-        const uint32_t K = min(seg_rows, T.rows - j * seg_rows);
-        const int r2 = lz4_seg_step((const uint32_t*)area, wbase, pc.lo, pc.hi, pc.end, s_seg[2 * ts],
-                                    s_seg[2 * ts + 1], K, buf + ts * (seg_rows + (1u << pl)), gl, G, in);
-        if (r2 && gl == 0) *s_err = r2;
-    }
+    lz4_segs(c.lz4_steps, tid, kPipeNC, glog, j0, nseg, T.rows, seg_rows, (const uint32_t*)area, wbase, pc.lo, pc.hi,
+             pc.end, s_seg, buf, 1u << pl, s_err);
     return (int)pl;
 }
 

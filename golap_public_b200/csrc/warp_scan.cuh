@@ -215,11 +215,11 @@ __device__ __noinline__ int ws_casc_rows(const uint8_t* __restrict__ pg, uint32_
 
 // The warp's per-segment LZ4 decode of a tile: segments j0 .. j0+nseg-1 of
 // the block that starts at address blk (blk_bytes compressed bytes; side
-// index entries e) into out (segment t at out + t * seg_rows), G lanes per
-// segment.  Returns 0 or kErrCorrupt (uniform).
+// index entries e) into out (segment t at out + t * seg_rows), groups of lanes
+// per segment.  Returns 0 or kErrCorrupt (uniform).
 __device__ __noinline__ int ws_lz4_rows(const uint8_t* blk, uint32_t blk_bytes, const uint32_t* e, uint32_t seg_shift,
                                         uint32_t rows, uint32_t r0, uint32_t n, uint32_t lo, uint32_t hi,
-                                        uint32_t* out, uint32_t lane) {
+                                        uint32_t* out, bool steps, uint32_t lane) {
     const uint32_t seg_rows = 1u << seg_shift;
     const uint32_t j0 = r0 >> seg_shift, nseg = (n + seg_rows - 1) >> seg_shift;
     // payload addresses keep the payload offsets' alignment modulo 16
@@ -227,20 +227,10 @@ __device__ __noinline__ int ws_lz4_rows(const uint8_t* blk, uint32_t blk_bytes, 
     const uint32_t* A = (const uint32_t*)a_wb;
     const uint32_t wbase = (uint32_t)(a_wb - (uintptr_t)blk);
     const uint32_t glog = seg_group_log2(nseg, 32);
-    const uint32_t G = 1u << glog;
-    const uint32_t gl = lane & (G - 1u);
     // the tile's compressed lines into L1 first, all in flight together
     for (uint32_t x = 128 * lane; x < hi - lo; x += 128 * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(A + x / 4));
     int err = 0;
-    for (uint32_t t0 = 0; t0 < nseg; t0 += (32u >> glog)) {
-        const uint32_t t = t0 + (lane >> glog);
-        const bool in = t < nseg;
-        const uint32_t j = j0 + (in ? t : 0u);
-        const uint32_t K = min(seg_rows, rows - j * seg_rows);
-        const uint32_t cp = __ldg(e + 2 * j), info = __ldg(e + 2 * j + 1);
-        if (lz4_seg_step(A, wbase, lo, hi, blk_bytes, cp, info, K, out + (in ? t : 0u) * seg_rows, gl, G, in))
-            err = kErrCorrupt;
-    }
+    lz4_segs(steps, lane, 32, glog, j0, nseg, rows, seg_rows, A, wbase, lo, hi, blk_bytes, e + 2 * j0, out, 0, &err);
     __syncwarp();
     return __any_sync(0xFFFFFFFFu, err != 0) ? kErrCorrupt : 0;
 }
@@ -366,7 +356,7 @@ __device__ __noinline__ int ws_decode_tile(const WsParams& P, const gx_dcol* s_c
         } else {
             const gx_dcol& col = s_cols[c];
             terr = ws_lz4_rows(cols[c].src, cols[c].bytes, col.seg + (size_t)2 * col.S * T.slot, col.seg_shift, T.rows,
-                               T.r0, T.n, cols[c].aux0, cols[c].aux1, buf, lane);
+                               T.r0, T.n, cols[c].aux0, cols[c].aux1, buf, col.lz4_steps != 0, lane);
         }
         __syncwarp();
         if (lane == 0) {

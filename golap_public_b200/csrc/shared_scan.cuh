@@ -678,10 +678,12 @@ __global__ void __launch_bounds__(NT, MINB) shared_scan_kernel(const __grid_cons
                             const int64_t val = prod ? (int64_t)v * c2 : diff ? (int64_t)v - c2 : (int64_t)v;
                             local += k ? val : 0;
                         }
-                    } else if (RPT <= 8 && (flags & GX_STEP_PROBE) && !last) {
-                        // probe of a join table: the chains of the thread's RPT rows are walked
-                        // together (ht_probe_rows), so that no row waits for another's (up to 8
-                        // rows per thread, where the registers allow)
+                    } else if (RPT <= 8 && (flags & GX_STEP_PROBE) && htlay != GX_HT_BUCKET && !last) {
+                        // probe of a dense or linear join table: the chains of the thread's RPT
+                        // rows are walked together (ht_probe_rows), so that no row waits for
+                        // another's (up to 8 rows per thread, where the registers allow).  Bucket
+                        // tables go row by row below, a repeated key without a probe: walked
+                        // together, batches over sorted dates took 8 % more
                         const uint64_t hdr = htlay == GX_HT_DENSE ? __ldg((const unsigned long long*)ht) : 0ull;
                         uint32_t vv[RPT], pay[RPT], m = 0;
 #pragma unroll

@@ -851,13 +851,22 @@ struct BuildPreds {
 
 // The counts of a build (inserted, duplicate, dropped rows) added up over the
 // CTA before they reach the table's counters: one atomic per thread on the
-// same word took longer than the inserts.  Called by all threads.
+// same word took longer than the inserts.  A few CTAs' warps add theirs
+// themselves (no barrier: 200 of 1000 rows inserted 3.0 us, 3.6 with it).
+// Called by all threads.
+constexpr uint32_t kHtFewCtas = 32;
+
 __device__ __forceinline__ void ht_count(uint32_t ins, uint32_t dup, uint32_t bad, unsigned long long* counters) {
     __shared__ uint32_t s_count[3];
-    if (threadIdx.x < 3) s_count[threadIdx.x] = 0;
-    __syncthreads();
     const uint32_t c[3] = {__reduce_add_sync(0xFFFFFFFFu, ins), __reduce_add_sync(0xFFFFFFFFu, dup),
                            __reduce_add_sync(0xFFFFFFFFu, bad)};
+    if (gridDim.x <= kHtFewCtas) {
+        if ((threadIdx.x & 31) < 3 && c[threadIdx.x & 31])
+            atomicAdd(&counters[threadIdx.x & 31], (unsigned long long)c[threadIdx.x & 31]);
+        return;
+    }
+    if (threadIdx.x < 3) s_count[threadIdx.x] = 0;
+    __syncthreads();
     if ((threadIdx.x & 31) < 3 && c[threadIdx.x & 31]) atomicAdd(&s_count[threadIdx.x & 31], c[threadIdx.x & 31]);
     __syncthreads();
     if (threadIdx.x < 3 && s_count[threadIdx.x]) atomicAdd(&counters[threadIdx.x], (unsigned long long)s_count[threadIdx.x]);
@@ -871,14 +880,14 @@ constexpr uint32_t kHtRows = 4;
 // The rows i0 + r * stride (r < kHtRows, below n) that pass the predicates
 // (bit r of the result) with their keys and table entries.  Every load is
 // issued before any is used; the reserved key counts as dropped.
+template <uint32_t R>
 __device__ __forceinline__ uint32_t ht_load_rows(const int32_t* keys, const int32_t* payload, uint64_t i0,
                                                  uint64_t stride, uint64_t n, const BuildPreds& preds,
-                                                 int32_t (&key)[kHtRows], unsigned long long (&e)[kHtRows],
-                                                 uint32_t& bad) {
+                                                 int32_t (&key)[R], unsigned long long (&e)[R], uint32_t& bad) {
     uint32_t m = 0;
-    int32_t pay[kHtRows];
+    int32_t pay[R];
 #pragma unroll
-    for (uint32_t r = 0; r < kHtRows; ++r) {
+    for (uint32_t r = 0; r < R; ++r) {
         const uint64_t i = i0 + r * stride;
         key[r] = kEmptyKey;
         pay[r] = (int32_t)i;
@@ -889,15 +898,15 @@ __device__ __forceinline__ uint32_t ht_load_rows(const int32_t* keys, const int3
         }
     }
     for (uint32_t k = 0; k < preds.n; ++k) {
-        int32_t x[kHtRows];
+        int32_t x[R];
 #pragma unroll
-        for (uint32_t r = 0; r < kHtRows; ++r) x[r] = (m >> r) & 1u ? __ldg(preds.p[k].col_dev + i0 + r * stride) : 0;
+        for (uint32_t r = 0; r < R; ++r) x[r] = (m >> r) & 1u ? __ldg(preds.p[k].col_dev + i0 + r * stride) : 0;
 #pragma unroll
-        for (uint32_t r = 0; r < kHtRows; ++r)
+        for (uint32_t r = 0; r < R; ++r)
             if (!(x[r] >= preds.p[k].lo && x[r] <= preds.p[k].hi)) m &= ~(1u << r);
     }
 #pragma unroll
-    for (uint32_t r = 0; r < kHtRows; ++r) {
+    for (uint32_t r = 0; r < R; ++r) {
         if (((m >> r) & 1u) && key[r] == kEmptyKey) {
             ++bad;
             m &= ~(1u << r);
@@ -909,24 +918,25 @@ __device__ __forceinline__ uint32_t ht_load_rows(const int32_t* keys, const int3
 
 // Linear-probing inserts of rows i0, i0 + stride, ... (< n) that pass the
 // predicates; counts inserted / duplicate / dropped rows.
+template <uint32_t R>
 __device__ __forceinline__ void ht_insert_rows(uint64_t* slots, uint32_t log2cap, const int32_t* keys,
                                                const int32_t* payload, uint64_t i0, uint64_t stride, uint64_t n,
                                                const BuildPreds& preds, uint32_t& ins, uint32_t& dup, uint32_t& bad) {
     const uint32_t mask = (1u << log2cap) - 1;
-    for (uint64_t i = i0; i < n; i += kHtRows * stride) {
-        int32_t key[kHtRows];
-        unsigned long long e[kHtRows];
+    for (uint64_t i = i0; i < n; i += R * stride) {
+        int32_t key[R];
+        unsigned long long e[R];
         uint32_t m = ht_load_rows(keys, payload, i, stride, n, preds, key, e, bad);
-        uint32_t s[kHtRows];
+        uint32_t s[R];
 #pragma unroll
-        for (uint32_t r = 0; r < kHtRows; ++r) s[r] = hash_key32(key[r], log2cap);
+        for (uint32_t r = 0; r < R; ++r) s[r] = hash_key32(key[r], log2cap);
         for (uint32_t t = 0; m && t <= mask; ++t) {  // one slot of every row left
-            unsigned long long old[kHtRows];
+            unsigned long long old[R];
 #pragma unroll
-            for (uint32_t r = 0; r < kHtRows; ++r)
+            for (uint32_t r = 0; r < R; ++r)
                 if ((m >> r) & 1u) old[r] = atomicCAS((unsigned long long*)slots + s[r], (unsigned long long)kEmptySlot, e[r]);
 #pragma unroll
-            for (uint32_t r = 0; r < kHtRows; ++r) {
+            for (uint32_t r = 0; r < R; ++r) {
                 if (!((m >> r) & 1u)) continue;
                 const bool free_slot = old[r] == (unsigned long long)kEmptySlot;
                 const bool same = !free_slot && (int32_t)(uint32_t)old[r] == key[r];
@@ -944,7 +954,7 @@ __global__ void ht_build_kernel(uint64_t* slots, uint32_t log2cap, const int32_t
                                 uint64_t n, const __grid_constant__ BuildPreds preds, unsigned long long* counters) {
     griddep_launch();
     uint32_t ins = 0, dup = 0, bad = 0;
-    ht_insert_rows(slots, log2cap, keys, payload, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
+    ht_insert_rows<kHtRows>(slots, log2cap, keys, payload, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
                    (uint64_t)gridDim.x * blockDim.x, n, preds, ins, dup, bad);
     ht_count(ins, dup, bad, counters);
 }
@@ -969,8 +979,13 @@ __global__ void __launch_bounds__(1024) ht_build_small_kernel(uint64_t* slots, u
     if (threadIdx.x < 4) counters[threadIdx.x] = 0;
     __syncthreads();
     uint32_t ins = 0, dup = 0, bad = 0;
-    ht_insert_rows(SMEM ? s_slots : slots, log2cap, keys, payload, threadIdx.x, blockDim.x, n, preds, ins, dup, bad);
-    ht_count(ins, dup, bad, counters);  // ends with the table complete
+    uint64_t* const tab = SMEM ? s_slots : slots;
+    if (n <= blockDim.x)  // (one row per thread: nothing to keep in flight beside it)
+        ht_insert_rows<1>(tab, log2cap, keys, payload, threadIdx.x, blockDim.x, n, preds, ins, dup, bad);
+    else
+        ht_insert_rows<kHtRows>(tab, log2cap, keys, payload, threadIdx.x, blockDim.x, n, preds, ins, dup, bad);
+    ht_count(ins, dup, bad, counters);
+    if (SMEM) __syncthreads();
     if (SMEM)
         for (uint32_t i = threadIdx.x; i < cap / 2; i += blockDim.x) ((ulonglong2*)slots)[i] = ((ulonglong2*)s_slots)[i];
 }
@@ -1067,44 +1082,62 @@ __global__ void ht_build_bucket_kernel(uint64_t* slots, uint32_t log2cap, const 
     ht_count(ins, dup, bad, counters);
 }
 
-// Probes of keys[0..n): four neighbouring keys per thread and step, one 16-byte
-// load and store where the arrays allow (vec), all four chains walked together
-// (16M probes of a 16 MB table: 137 us one key at a time, 90 us; bound by the
-// random sectors read from L2).
+// Probes of keys[0..n): a warp takes 32 R keys at a time, R per lane, their
+// chains walked together while the next keys are read; four per lane as one
+// 16-byte load and store where the arrays allow (vec), else 32 apart (lane by
+// lane, so that a warp's accesses stay whole lines).  16M probes of a 16 MB
+// table, bound by the random sectors read from L2: 137 us one key at a time, 88
+// us; of 30K entries through unaligned arrays 46 and 35 us.  Few keys
+// (kHtProbeOne; 16 times as many when no hits are counted, an atomic per warp)
+// are one per lane, which is all latency: 1000 probes 2.6 us at four, 2.1 at
+// one; 100,000 counted ones 2.8 and 3.9, not counted 2.6 and 2.4.
+constexpr uint64_t kHtProbeOne = 1u << 14;
+template <uint32_t R>
 __global__ void __launch_bounds__(256) ht_probe_kernel(const uint64_t* slots, uint32_t log2cap, uint32_t layout,
                                                        const int32_t* keys, uint64_t n, int32_t* out,
                                                        unsigned long long* hits, uint32_t vec) {
     const uint64_t pol = ws_policy_keep();
     const uint64_t hdr = layout == GX_HT_DENSE ? __ldg((const unsigned long long*)slots) : 0ull;
+    const uint32_t lane = threadIdx.x & 31;
     unsigned long long h = 0;
-    const uint64_t stride = 4ull * gridDim.x * blockDim.x;
-    for (uint64_t i = 4 * (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x); i < n; i += stride) {
-        uint32_t v[4] = {(uint32_t)kEmptyKey, (uint32_t)kEmptyKey, (uint32_t)kEmptyKey, (uint32_t)kEmptyKey};
-        uint32_t pay[4] = {0, 0, 0, 0};
-        const bool whole = vec && i + 4 <= n;
-        if (whole) {
-            const uint4 x = __ldcs((const uint4*)(keys + i));
+    const uint64_t stride = (uint64_t)R * gridDim.x * blockDim.x;
+    // the lane's keys of the warp's 32 R keys from c on
+    auto load = [&](uint64_t c, uint32_t (&v)[R]) {
+        if (R == 4 && vec && c + 128 <= n) {
+            const uint4 x = __ldcs((const uint4*)(keys + c) + lane);
             v[0] = x.x;
-            v[1] = x.y;
-            v[2] = x.z;
-            v[3] = x.w;
+            v[1 % R] = x.y;
+            v[2 % R] = x.z;
+            v[3 % R] = x.w;
         } else {
 #pragma unroll
-            for (uint32_t r = 0; r < 4; ++r)
-                if (i + r < n) v[r] = (uint32_t)__ldg(keys + i + r);
+            for (uint32_t r = 0; r < R; ++r)
+                v[r] = c + 32 * r + lane < n ? (uint32_t)__ldg(keys + c + 32 * r + lane) : (uint32_t)kEmptyKey;
         }
-        const uint32_t m = ht_probe_rows<4>(slots, log2cap, layout, hdr, v, 15u, pay, pol);
+    };
+    uint32_t nx[R];
+    uint64_t c = R * (blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u));
+    if (c < n) load(c, nx);
+    for (; c < n; c += stride) {
+        uint32_t v[R], pay[R];
+#pragma unroll
+        for (uint32_t r = 0; r < R; ++r) {
+            v[r] = nx[r];
+            pay[r] = 0;
+        }
+        if (c + stride < n) load(c + stride, nx);  // the next keys while these are probed
+        const uint32_t m = ht_probe_rows<R>(slots, log2cap, layout, hdr, v, (1u << R) - 1u, pay, pol);
         h += __popc(m);
         if (out) {
 #pragma unroll
-            for (uint32_t r = 0; r < 4; ++r)
+            for (uint32_t r = 0; r < R; ++r)
                 if (!((m >> r) & 1u)) pay[r] = (uint32_t)INT32_MIN;
-            if (whole) {
-                __stcs((uint4*)(out + i), make_uint4(pay[0], pay[1], pay[2], pay[3]));
+            if (R == 4 && vec && c + 128 <= n) {
+                __stcs((uint4*)(out + c) + lane, make_uint4(pay[0], pay[1 % R], pay[2 % R], pay[3 % R]));
             } else {
 #pragma unroll
-                for (uint32_t r = 0; r < 4; ++r)
-                    if (i + r < n) out[i + r] = (int32_t)pay[r];
+                for (uint32_t r = 0; r < R; ++r)
+                    if (c + 32 * r + lane < n) out[c + 32 * r + lane] = (int32_t)pay[r];
             }
         }
     }
@@ -1715,9 +1748,14 @@ gx_status gx_hashtable_probe(const gx_hashtable* ht, const int32_t* keys_dev, ui
                              uint64_t* hits_dev, void* stream) {
     if (!ht || (!keys_dev && n)) return set_error(GX_ERR_INVALID, "gx_hashtable_probe: bad args");
     if (n == 0) return GX_OK;
+    cudaStream_t s = (cudaStream_t)stream;
     const uint32_t vec = (((uintptr_t)keys_dev | (uintptr_t)payload_out_dev) & 15u) == 0;
-    ht_probe_kernel<<<(unsigned)std::min<uint64_t>(8 * sm_count(), (n + 1023) / 1024), 256, 0, (cudaStream_t)stream>>>(
-        ht->slots, ht->log2cap, ht->layout, keys_dev, n, payload_out_dev, (unsigned long long*)hits_dev, vec);
+    if (n <= (hits_dev ? kHtProbeOne : 16 * kHtProbeOne))
+        ht_probe_kernel<1><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+            ht->slots, ht->log2cap, ht->layout, keys_dev, n, payload_out_dev, (unsigned long long*)hits_dev, vec);
+    else
+        ht_probe_kernel<4><<<(unsigned)std::min<uint64_t>(8 * sm_count(), (n + 1023) / 1024), 256, 0, s>>>(
+            ht->slots, ht->log2cap, ht->layout, keys_dev, n, payload_out_dev, (unsigned long long*)hits_dev, vec);
     GX_CK(cudaGetLastError());
     return GX_OK;
 }

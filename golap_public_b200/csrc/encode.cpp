@@ -40,6 +40,7 @@ inline uint32_t ext_bytes(uint32_t len) {  // extension bytes for a 4-bit field 
 struct SeqEmitter {
     std::vector<uint8_t>& out;
     uint32_t n_seq = 0;     // sequences emitted
+    uint32_t n_short = 0;   // ... with at most one literal length byte and no match length byte after the token
     size_t base;            // offset of the block start in out
     const uint8_t* bytes;   // input block as bytes
     uint32_t* seg;          // 2*S entries
@@ -57,6 +58,7 @@ struct SeqEmitter {
         const uint32_t Mb = mlen_w * 4;
         const uint32_t mnib = has_match ? std::min<uint32_t>(Mb - 4, 15) : 0;
         const uint32_t lit0 = tp + 1 + ext_bytes(Lb);
+        n_short += mnib < 15 && ext_bytes(Lb) <= 1;
         if (n_seq == 1 && Lb > 0) {
             // entry 0 resumes inside the block's first literal run (not at its token),
             // so a tile at the block start whose rows are literals is a plain byte range
@@ -105,19 +107,20 @@ struct SeqEmitter {
 // current segment.
 size_t lz4_encode_block(const int32_t* vals, uint32_t W, uint32_t S, uint32_t seg_rows,
                         uint32_t min_match, uint32_t depth, std::vector<uint8_t>& out,
-                        uint32_t* seg, uint32_t* n_seq) {
+                        uint32_t* seg, uint32_t* n_seq, uint32_t* n_short) {
     constexpr uint32_t HB = 14;
     const size_t base = out.size();
     std::vector<uint32_t> bound(S + 1);
     for (uint32_t j = 0; j <= S; ++j) bound[j] = std::min<uint64_t>((uint64_t)j * seg_rows, W);
     seg[0] = 0;
     seg[1] = 0;
-    SeqEmitter em{out, 0, base, (const uint8_t*)vals, seg, bound.data(), S};
+    SeqEmitter em{out, 0, 0, base, (const uint8_t*)vals, seg, bound.data(), S};
     const uint32_t min_w = std::max<uint32_t>(1, (min_match + 3) / 4);
     if (min_w >= W) {  // no match can be long enough: the block is one literal run
         em.emit(0, W, false, 0, 0);
         em.finish(W);
         if (n_seq) *n_seq = em.n_seq;
+        if (n_short) *n_short = em.n_short;
         return out.size() - base;
     }
     std::vector<int32_t> head(1u << HB, -1);
@@ -167,6 +170,7 @@ size_t lz4_encode_block(const int32_t* vals, uint32_t W, uint32_t S, uint32_t se
     em.emit(anchor, W, false, 0, 0);
     em.finish(W);
     if (n_seq) *n_seq = em.n_seq;
+    if (n_short) *n_short = em.n_short;
     return out.size() - base;
 }
 
@@ -412,7 +416,7 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
     if (threads == 0) threads = std::max(1u, std::thread::hardware_concurrency());
     threads = std::min<uint32_t>(threads, std::max<uint32_t>(1, col->n_slots));
     std::vector<std::vector<uint8_t>> bufs(threads);
-    std::atomic<uint64_t> seqs{0};
+    std::atomic<uint64_t> seqs{0}, short_seqs{0};
     std::atomic<bool> overflow{false}, all_simple{codec == GX_CODEC_CASCADED};
     std::vector<std::vector<uint64_t>> local_off(threads);
     auto work = [&](uint32_t t) {
@@ -446,13 +450,14 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
                 buf.insert(buf.end(), (const uint8_t*)(vals + r0), (const uint8_t*)(vals + r0 + rows));
                 used = (size_t)rows * 4;
             } else if (codec == GX_CODEC_LZ4) {
-                uint32_t tmp_seg[2 * kMaxSegments], n_seq = 0;
+                uint32_t tmp_seg[2 * kMaxSegments], n_seq = 0, n_short = 0;
                 lz4_tmp.clear();
                 used = min_match ? lz4_encode_block(vals + r0, rows, S, rows_per_block / S, min_match, depth, lz4_tmp,
-                                                    tmp_seg, &n_seq)
+                                                    tmp_seg, &n_seq, &n_short)
                                  : lz4_encode_block_auto(vals + r0, rows, S, rows_per_block / S, depth, lz4_tmp,
                                                          tmp_seg);
                 seqs += n_seq;
+                short_seqs += n_short;
                 if (used + 16 > kStageBytes) overflow = true;  // cannot happen for <= 16384 int32 rows
                 if (S > 1) std::memcpy(&col->seg[(size_t)2 * S * s], tmp_seg, 8 * S);
                 // place the block so that its first literal byte is 16-byte aligned
@@ -492,6 +497,7 @@ int column_encode(const int32_t* vals, uint64_t n_rows, uint32_t codec, uint32_t
     for (auto& th : pool) th.join();
     col->casc_simple = all_simple;
     col->lz4_seqs = seqs;
+    col->lz4_short = short_seqs;
     if (overflow) return set_error(GX_ERR_INVALID, "an LZ4 block exceeds the %u-byte staging buffer", kStageBytes);
     // the per-thread buffers in thread order, each copied by its own thread
     std::vector<uint64_t> shift(threads + 1, 0);

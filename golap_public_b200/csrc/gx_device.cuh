@@ -352,11 +352,13 @@ __device__ __forceinline__ int lz4_seg_step(const uint32_t* __restrict__ A, uint
     return active && !ok ? kErrCorrupt : 0;
 }
 
-// Which of the two a column takes: groups in step (gx_dcol::lz4_steps) from three
-// sequences to 16 rows on.  Measured on both sides of that line, groups in step
-// against each on its own (time of decompressing / a pipelined / a shared scan
-// of 8M rows): 0.24 to 0.78 sequences per row 0.88 to 1.02 / 0.75 to 0.84 / 0.80
-// to 0.96; 0.02 to 0.13 per row 0.97 to 1.14 / 1.05 to 1.12 / 1.03 to 1.09.
+// Which of the two a column takes: groups in step (gx_dcol::lz4_steps) when at
+// least three in four of its sequences fit a round of short ones (the groups of
+// a warp have to have one at the same time), whatever the number of sequences.
+// Measured on both sides of that line, groups in step against each on its own
+// (time of decompressing / a pipelined / a shared scan of 8M rows): 90 to 100 %
+// short 0.88 to 1.02 / 0.75 to 0.84 / 0.80 to 0.96; up to 23 % short 0.96 to
+// 1.16 / 1.02 to 1.12 / 1.02 to 1.09.
 enum class LzGroups { kEither, kAlone, kInStep };  // the decoders an instance holds
 
 // nseg segments (block segments j0 ..; entries at seg) by the tid-th of NT

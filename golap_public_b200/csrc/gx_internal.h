@@ -137,7 +137,7 @@ struct gx_dcol {
     uint32_t n_slots;           // n_chunks * blocks_per_chunk
     uint64_t payload_bytes;     // size of the payload allocation
     uint32_t host_mapped;       // payload lives in pinned host memory (no TMA staging)
-    uint32_t lz4_steps;         // LZ4 with segments: many short sequences (LzGroups in gx_device.cuh)
+    uint32_t lz4_steps;         // LZ4 with segments: mostly short sequences (LzGroups in gx_device.cuh)
 };
 
 // Bit-packed stream reader: element i of width w (0..32).
@@ -200,7 +200,8 @@ struct gx_column {
     uint32_t* d_bloom = nullptr;
     // LZ4: every block is one 16-byte aligned literal run (-1 = not known yet)
     mutable int lz4_direct = -1;
-    uint64_t lz4_seqs = 0;     // LZ4 with a fixed minimum match: sequences of the column, known when encoded
+    uint64_t lz4_seqs = 0;     // LZ4 with a fixed minimum match: sequences of the column, known when encoded,
+    uint64_t lz4_short = 0;    // and those a round of lz4_seg_step takes whole
     bool casc_simple = false;  // cascaded: every page is simple (casc_page_simple), known when encoded
     int32_t* d_bmins = nullptr;
     int32_t* d_bmaxs = nullptr;
@@ -228,7 +229,7 @@ struct gx_column {
         v.n_slots = n_slots;
         v.payload_bytes = host_pending ? dev_payload_bytes : payload.size();
         v.host_mapped = residency == 2 ? 1u : 0u;
-        v.lz4_steps = lz4_seqs * 16 >= n_rows * 3 ? 1u : 0u;
+        v.lz4_steps = lz4_seqs && lz4_short * 4 >= lz4_seqs * 3 ? 1u : 0u;
         return v;
     }
 };
@@ -245,7 +246,8 @@ int host_payload(const gx_column* col);
 // block; returns the compressed size, appends S {comp_pos, info} pairs to seg.
 size_t lz4_encode_block(const int32_t* vals, uint32_t rows, uint32_t S, uint32_t seg_rows,
                         uint32_t min_match, uint32_t depth, std::vector<uint8_t>& out,
-                        uint32_t* seg_entries, uint32_t* n_seq);
+                        uint32_t* seg_entries, uint32_t* n_seq,
+                        uint32_t* n_short = nullptr);
 size_t lz4_encode_block_auto(const int32_t* vals, uint32_t rows, uint32_t S, uint32_t seg_rows, uint32_t depth,
                              std::vector<uint8_t>& out, uint32_t* seg_entries);
 size_t casc_encode_page(const int32_t* vals, uint32_t rows, bool allow_rle, bool allow_delta,

@@ -246,6 +246,7 @@ struct __align__(16) WsTile {
 constexpr uint32_t kWsDecode = 1u << 29;     // a column needs a decode, or is corrupt
 constexpr uint32_t kWsDead = 1u << 30;       // a constant step drops every row
 constexpr uint32_t kWsMixed = 1u << 31;      // a column is neither direct nor a loose step's that is not packed
+constexpr uint32_t kWsHard = 1u << 28;       // ... nor decoded
 static_assert(sizeof(WsTile) == 32, "tile records of 8 words");
 
 // How one column of one tile is read.
@@ -526,6 +527,7 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
         if (dir_ok && d_bytes == rows * 4 && (d_off & 15u) == 0) {
             C.mode = kWmDirect;
             C.src = blk + 4ull * r0;
+            C.aux0 = 31;
         }
     } else if (col.codec == GX_CODEC_LZ4) {
         const uint32_t sr = 1u << col.seg_shift;
@@ -540,6 +542,7 @@ __device__ __forceinline__ WsCol ws_column(const WsParams& P, const gx_dcol& col
                 if (lit && ((d_off + e0) & 15u) == 0) {
                     C.mode = kWmDirect;
                     C.src = blk + e0;
+                    C.aux0 = 31;
                 } else if (P.buf_of[c] != kWsNone) {
                     C.mode = kWmLz4;
                     C.src = blk;
@@ -697,7 +700,7 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
                                                uint32_t lane) {
     const ShQuery& Q = P.q;
     const uint32_t cl = P.col_log2, q = lane >> cl, s = lane & ((1u << cl) - 1u);
-    bool isc = false, ok = true, bad = false, mixed = false, dec = false, digits = false;
+    bool isc = false, ok = true, bad = false, mixed = false, hard = false, dec = false, digits = false;
     if (((vm >> q) & 1u) && s < P.n_cols) {  // as a column
         const uint32_t m = cols[lane].mode;
         dec = m == kWmLz4 || m == kWmCasc || m == kWmBad;
@@ -709,6 +712,7 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
         mixed = c.mode != kWmDirect &&
                 (c.mode == kWmPack || !ws_loose_step(s, Q.n_steps, (st.flags & GX_STEP_PROBE) != 0,
                                                      (st.flags & GX_STEP_CARRY) != 0));
+        hard = mixed && c.mode != kWmLz4 && c.mode != kWmCasc;
         if (isc) {
             const int32_t v = c.cval;
             int32_t pp = v;
@@ -729,15 +733,16 @@ __device__ __forceinline__ void ws_const_steps(const WsParams& P, uint32_t vm, W
     const uint32_t digs = (__ballot_sync(0xFFFFFFFFu, digits) >> sh) & m0;
     const uint32_t decs = (__ballot_sync(0xFFFFFFFFu, dec) >> sh) & m0;
     const uint32_t mixes = (__ballot_sync(0xFFFFFFFFu, mixed) >> sh) & m0;
+    const uint32_t hards = (__ballot_sync(0xFFFFFFFFu, hard) >> sh) & m0;
     if (s == 0 && ((vm >> q) & 1u)) {
-        uint32_t f = cst | (mixes ? kWsMixed : 0u) | (fails ? kWsDead : 0u);
+        uint32_t f = cst | (mixes ? kWsMixed : 0u) | (hards ? kWsHard : 0u) | (fails ? kWsDead : 0u);
         // a digit out of range is an error for rows alive at its step: its tile's
         // steps are taken row by row (a step over rows before it may have dropped
         // them) unless a constant step before it drops the tile.  Run-time plans
         // also look at the digits of rows before they let a constant step drop
         // them; the compile-time ones leave such a tile unread
         const uint32_t before = fails ? (1u << (__ffs(fails) - 1)) - 1u : m0;
-        if (((fails ? digs : bads) & before) != 0) f = kWsMixed;
+        if (((fails ? digs : bads) & before) != 0) f = kWsMixed | kWsHard;
         f |= decs ? kWsDecode : 0u;
         tiles[q].steps = f;
     }
@@ -819,6 +824,15 @@ __device__ __forceinline__ uint4 ws_decoded(const WsCol& d, uint32_t row) {
     return *(const uint4*)(d.src + 4 * (row + ((row >> d.aux0) << 2)));
 }
 
+// Tile rows row .. row + 3 of a direct or decoded column (generic address).
+__device__ __forceinline__ uint4 ws_ld_any(const WsCol& d, uint32_t row) {
+    uint4 v;
+    asm volatile("ld.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(d.src + 4 * (row + ((row >> d.aux0) << 2))));
+    return v;
+}
+
 // Tile rows row .. row + 3 of a column, however it is read.
 __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
     const uint32_t mode = d.mode;
@@ -830,25 +844,30 @@ __device__ __forceinline__ uint4 ws_quad(const WsCol& d, uint32_t row) {
     return ws_decoded(d, row);  // kWmRows
 }
 
+enum class WsForm { kAny, kFlat, kRows };
+
 // Tile rows [a, b) evaluated through the plan's steps, H 128-row groups at a
 // time (a is a multiple of kWsPartRows): the lane's rows of group j are
 // 128 j + 4 lane + i (i < 4), row r = 4 h + i of the batch; bit r of m is its
 // mask.  A compile-time signature loads all columns of the batch before any
 // is used and unrolls its steps: up to the last probe step by step, the
 // filters after it and the aggregate row by row, where a row's mask is a
-// predicate.  Run-time plans with a group key load a column at its step.  FLAT:
+// predicate.  Run-time plans with a group key load a column at its step.  kFlat:
 // [a, b) is whole batches and every column is direct or a loose step's that is
 // not packed (a sorted date), so that a batch's loads are unconditional and all
-// in flight together.  Steps over constant columns were decided by
+// in flight together; kRows: the same with decoded columns among them, every
+// quad from a generic address (as kAny, where a quad's read mode is looked up
+// first, four batches of a tile took 14,000 cycles, which a pruned scan of a few
+// such tiles waits for).  Steps over constant columns were decided by
 // ws_const_steps.
 // Returns the scalar part; grouped sums go to the CTA's group table through
 // the warp's queue.
-template <uint32_t SIG, bool FLAT>
+template <uint32_t SIG, WsForm FORM>
 __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, uint32_t cst, const uint32_t* sdig,
                                            uint32_t a, uint32_t b, uint32_t* tkey, WsQueue* wq, uint32_t& qn,
                                            uint64_t pol_keep, const uint64_t* s_hdr,
                                            uint32_t lane) {
-    constexpr bool RT = kWsRunTime<SIG>;
+    constexpr bool RT = kWsRunTime<SIG>, FLAT = FORM != WsForm::kAny, ROWS = FORM == WsForm::kRows;
     constexpr bool GR = ((SIG >> 6) & 1) != 0;  // grouped: the queue holds one row group
     constexpr uint32_t H = GR ? 1 : kWsEvalGroups;
     constexpr uint32_t R = 4 * H;
@@ -862,7 +881,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
     if (!RT) {
 #pragma unroll
         for (uint32_t s = 0; s < NS; ++s) {
-            src[s] = FLAT ? cols[Q.steps[s].col].src + (a + 4 * lane) * 4 : nullptr;
+            src[s] = FLAT && !ROWS ? cols[Q.steps[s].col].src + (a + 4 * lane) * 4 : nullptr;
             if (s + 1 > PE && ((SIG >> (7 + 4 * s)) & kWkF) && Q.steps[s].lo > Q.steps[s].hi) some = 0;
         }
     }
@@ -896,6 +915,8 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
                         const WsCol& d = cols[Q.steps[s].col];
                         if (loose && !skip && d.mode == kWmRuns2)
                             x = ws_runs2(d, row + kWsBatch * h);
+                        else if (ROWS && !skip)
+                            x = ws_ld_any(d, row + kWsBatch * h);
                         else if (loose && !skip && d.mode == kWmRows)
                             x = ws_decoded(d, row + kWsBatch * h);
                         else if (!skip)
@@ -905,7 +926,7 @@ __device__ __forceinline__ int64_t ws_eval(const ShQuery& Q, const WsCol* cols, 
                     }
                     ws_put(w[s], h, x);
                 }
-                if (FLAT) src[s] += H * kWsBatch * 4;
+                if (FLAT && !ROWS) src[s] += H * kWsBatch * 4;
             }
             if (!FLAT) {
 #pragma unroll
@@ -1162,15 +1183,20 @@ __device__ __forceinline__ int64_t ws_eval_steps(const ShQuery& Q, const WsCol* 
     return acc;
 }
 
-// The general evaluator out of line: ragged tiles, columns that are not
-// direct, run-time plans.
+// The signatures with a kRows evaluator: scalar ones.  (One more instance in the
+// kernel of the grouped star join cost it 2.6 %.)
 template <uint32_t SIG>
+constexpr bool kWsRows = !kWsRunTime<SIG> && ((SIG >> 6) & 1) == 0;
+
+// The other evaluators out of line: tiles with decoded columns; ragged tiles,
+// other columns that are not direct, run-time plans.
+template <uint32_t SIG, WsForm FORM>
 __device__ __noinline__ int64_t ws_eval_any(const ShQuery& Q, const WsCol* cols, uint32_t cst, const uint32_t* sdig,
                                             uint32_t a, uint32_t b, uint32_t* tkey, WsQueue* wq, uint32_t* qn,
                                             uint64_t pol_keep, const uint64_t* s_hdr,
                                             uint32_t lane) {
     uint32_t n = *qn;
-    const int64_t acc = ws_eval<SIG, false>(Q, cols, cst, sdig, a, b, tkey, wq, n, pol_keep, s_hdr, lane);
+    const int64_t acc = ws_eval<SIG, FORM>(Q, cols, cst, sdig, a, b, tkey, wq, n, pol_keep, s_hdr, lane);
     *qn = n;
     return acc;
 }
@@ -1330,10 +1356,14 @@ __global__ void __launch_bounds__(kWsNT, ws_ctas(SIG)) warp_scan_kernel(const __
                 if constexpr (SIG == kSigRt)
                     local += ws_eval_steps(Q, cols, st, T.a, T.b, pol_keep, whdr, lane);
                 else if (!kWsRunTime<SIG> && !(st & kWsMixed) && ((T.b - T.a) & (kWsPartRows - 1u)) == 0)
-                    local += ws_eval<SIG, !kWsRunTime<SIG>>(Q, cols, st, dig, T.a, T.b, tkey, wq, qn, pol_keep, whdr,
-                                                            lane);
+                    local += ws_eval<SIG, kWsRunTime<SIG> ? WsForm::kAny : WsForm::kFlat>(
+                        Q, cols, st, dig, T.a, T.b, tkey, wq, qn, pol_keep, whdr, lane);
+                else if (kWsRows<SIG> && !(st & kWsHard) && ((T.b - T.a) & (kWsPartRows - 1u)) == 0)
+                    local += ws_eval_any<SIG, kWsRows<SIG> ? WsForm::kRows : WsForm::kAny>(
+                        Q, cols, st, dig, T.a, T.b, tkey, wq, &qn, pol_keep, whdr, lane);
                 else
-                    local += ws_eval_any<SIG>(Q, cols, st, dig, T.a, T.b, tkey, wq, &qn, pol_keep, whdr, lane);
+                    local += ws_eval_any<SIG, WsForm::kAny>(Q, cols, st, dig, T.a, T.b, tkey, wq, &qn, pol_keep, whdr,
+                                                            lane);
             }
             __syncwarp();  // every lane is done with the tile's buffers and records before they are overwritten
         }

@@ -2388,7 +2388,7 @@ static gx_status scan_launch_warp(const gx_scan_plan* plan, const QueryDesc& qd,
               (c->codec == GX_CODEC_CASCADED && c->casc_simple))) {
             if (c->codec == GX_CODEC_LZ4) cut_tiles = false;
             // a lane per segment: at least three sequences to eight rows (1.5 words a sequence, Q1
-            // over 10M rows: 320 us, 570 with lz4_seg_step; 4 words, 6M rows: 250 and 168)
+            // over 10M rows: 302 us, 570 with lz4_seg_step; 4 words, 6M rows: 250 and 168)
             if (c->codec == GX_CODEC_LZ4 && c->seg_shift >= kWsLaneShift0 && c->seg_shift <= kWsLaneShift1 &&
                 c->lz4_seqs * 8 >= c->n_rows * 3) {
                 P.lane_cols |= 1u << i;

@@ -155,17 +155,6 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* m, uint32_t phase, 
     return false;
 }
 
-// Named-barrier OR-vote of the consumer warps.
-__device__ __forceinline__ bool pipe_any(bool p) {
-    uint32_t r;
-    asm volatile(
-        "{\n .reg .pred a, b;\n setp.ne.u32 a, %1, 0;\n bar.red.or.pred b, %2, %3, a;\n selp.u32 %0, 1, 0, b;\n}"
-        : "=r"(r)
-        : "r"((uint32_t)p), "n"(kPipeBar), "n"(kPipeNC)
-        : "memory");
-    return r != 0;
-}
-
 // Chunk-level keep of the query (keep_in and every prune predicate's chunk
 // min/max: the reference's pruning granularity).
 __device__ __forceinline__ bool pipe_chunk_keep(const ShQuery& Q, uint32_t chunk) {

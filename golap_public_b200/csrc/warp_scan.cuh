@@ -9,9 +9,10 @@
 // (core/metadata.cuh:638-658) and the per-chunk worker loop of
 // usecases/ssb/queries/01.hpp:350-424 folded into the same launch.
 //
-// Every warp is an independent worker: after one block-wide barrier at the
+// Every warp is an independent worker: after two block-wide barriers at the
 // start (chunk keep bits of the launch and their prefix counts, computed by
-// each CTA) no warp waits for another.  The 1024-row tiles of the surviving
+// each CTA) no warp waits for another; grouped plans have one more at the end,
+// before the CTA's group table is flushed.  The 1024-row tiles of the surviving
 // chunks form a dense rank space; warp w of the grid takes tiles w, w + W,
 // w + 2W, ... (W warps), and the tiles of the last, incomplete round are cut
 // into 256- or 512-row parts when there are warps to spare (so a pruned scan
@@ -33,7 +34,8 @@
 //     128 rows (4 consecutive rows per lane, one 16-byte load per column).
 //     Plans of the SSB shapes run a compile-time evaluator selected by their
 //     signature (all values of its row groups loaded before any is used);
-//     other plans the same evaluator with its steps read at run time.
+//     other plans read their steps at run time: with a group key in the same
+//     evaluator, without one step by step over the tile (ws_eval_steps).
 // Scalar sums stay in registers; grouped rows are collected per warp and
 // added, 32 at a time, to the CTA's group table in shared memory (keys that
 // find no slot go to the global table), flushed when the CTA is done.
@@ -765,9 +767,9 @@ constexpr uint32_t kSigQ1 = ws_sig(4, GX_AGG_SUM_PRODUCT, false, kWkP, kWkF | kW
 constexpr uint32_t kSigQ3 = ws_sig(4, GX_AGG_SUM, true, kWkP | kWkD, kWkP | kWkD, kWkP | kWkD, 0);
 // pipeline_q2: part probe (brand digit), supplier probe, date probe (year digit), revenue grouped
 constexpr uint32_t kSigQ2 = ws_sig(4, GX_AGG_SUM, true, kWkP | kWkD, kWkP, kWkP | kWkD, 0);
-// pipeline_q4: customer (nation digit), supplier, date (year digit), part probes, supplycost carried, profit grouped
 // a group-by of one column over a range of another (dates): value grouped by a digit
 constexpr uint32_t kSigGroup = ws_sig(3, GX_AGG_SUM, true, kWkF, kWkD, 0);
+// pipeline_q4: customer (nation digit), supplier, date (year digit), part probes, supplycost carried, profit grouped
 constexpr uint32_t kSigQ4 = ws_sig(6, GX_AGG_SUM_DIFF, true, kWkP | kWkD, kWkP, kWkP | kWkD, kWkP, kWkC, 0);
 
 // The steps of a signature that run step by step: up to the last probe, and

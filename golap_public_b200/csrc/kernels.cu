@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(256) ht_probe_kernel(const uint64_t* slots, ui
         } else {
 #pragma unroll
             for (uint32_t r = 0; r < R; ++r)
-                v[r] = c + 32 * r + lane < n ? (uint32_t)__ldg(keys + c + 32 * r + lane) : (uint32_t)kEmptyKey;
+                v[r] = c + 32 * r + lane < n ? (uint32_t)__ldcs(keys + c + 32 * r + lane) : (uint32_t)kEmptyKey;
         }
     };
     uint32_t nx[R];
